@@ -15,6 +15,7 @@
 #include "devmem.h"
 #include "match.h"
 #include "pr_launch.h"
+#include "resident.h"
 #include "wbpr_internal.h"
 
 using namespace wbpr_dev;
@@ -179,6 +180,10 @@ struct wbpr_graph {
   int* mt_cy = nullptr;
   int* mt_lmin = nullptr;
   MCtl* mt_ctl = nullptr;
+  // resident solver: blocks of the cluster whose shared memory holds the
+  // graph (0: none does), and what its launch reports
+  int res_cluster = 0;
+  ResOut* res_out = nullptr;
   int64_t bytes = 0;
   std::vector<void*> allocs;
 };
@@ -1414,6 +1419,7 @@ wbpr_status create_impl(const wbpr_csr* in, wbpr_layout layout, wbpr_graph** out
   TRYC(cudaEventCreate(&g->ev3));
   const int n = g->n;
   TRY(build_device(g, in));
+  g->res_cluster = resident_cluster(g->n, g->total_deg);
   int** vec[] = {&g->h, &g->e, &g->rl_min, &g->rl_left, &g->lq[0], &g->lq[1], &g->hq[0], &g->hq[1],
                  &g->esnap, &g->dmin0,
                  &g->qraw, &g->fr[0], &g->fr[1], &g->fr[2], &g->vlab};
@@ -1526,6 +1532,7 @@ struct RunCfg {
   int greedy;
   int bfs_alpha;
   int gr_plateau;
+  bool resident;  // no knob of the persistent kernel is set: the resident solver may take it
   bool matching;  // the matching kernel may take unit-capacity bipartite networks
   long long max_rounds;
   unsigned long long budget_ns;
@@ -1625,7 +1632,73 @@ wbpr_status run_kernel(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch
   return WBPR_OK;
 }
 
+bool use_resident(const wbpr_graph* g, const RunCfg& rc) { return rc.resident && !rc.term && g->res_cluster > 0; }
+
+// One launch of the resident solver.  *fits is cleared (and the handle's
+// cluster size raised, or set to 0) when a block's share of the graph is
+// larger than its shared memory; nothing has changed then.
+wbpr_status run_resident(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch_ms, int* flow, bool* fits) {
+  *fits = true;
+  if (!g->res_out) {
+    wbpr_status st = dalloc(g, &g->res_out, 1);
+    if (st) return st;
+  }
+  ResParams p{};
+  p.in.n = g->n;
+  p.in.mode = rc.mode;
+  p.in.s = rc.mode == kModeBfsOnly ? rc.bfs_excl : rc.s;
+  p.in.t = rc.mode == kModeBfsOnly ? rc.bfs_root : rc.t;
+  p.in.dir = rc.bfs_dir;
+  if (g->layout == WBPR_LAYOUT_BCSR) {
+    p.in.row = g->row;
+    p.in.arc = g->arc;
+    p.in.arx = g->arx;
+  } else {
+    p.in.frow = g->frow;
+    p.in.farc = g->farc;
+    p.in.fcb = g->fcb;
+    p.in.fcap = g->fcap;
+    p.in.rrow = g->rrow;
+    p.in.rarc = g->rarc;
+  }
+  p.in.lab = rc.lab ? rc.lab : g->h;
+  p.in.e = g->e;
+  p.out = g->res_out;
+  p.max_rounds = rc.max_rounds;
+  p.budget_ns = rc.budget_ns;
+  ResOut h;
+  for (;;) {
+    if (launch_ms) CK(cudaEventRecord(g->ev2, g->stream));
+    if (launch_resident(p, g->avg_deg < 20 ? 8 : 32, g->res_cluster, g->stream) != cudaSuccess) {
+      cudaGetLastError();  // no such cluster on this device: the persistent kernel takes the graph
+      g->res_cluster = 0;
+      *fits = false;
+      return WBPR_OK;
+    }
+    if (launch_ms) CK(cudaEventRecord(g->ev3, g->stream));
+    CK(cudaMemcpyAsync(&h, g->res_out, sizeof(h), cudaMemcpyDeviceToHost, g->stream));
+    CK(cudaStreamSynchronize(g->stream));
+    if (h.err != kResNoFit) break;
+    g->res_cluster = g->res_cluster < kResMaxCluster ? 2 * g->res_cluster : 0;
+    if (!g->res_cluster) {
+      *fits = false;
+      return WBPR_OK;
+    }
+  }
+  if (rc.mode != kModeBfsOnly) g->full_reset = true;  // its pushes are not in the undo log
+  if (launch_ms) CK(cudaEventElapsedTime(launch_ms, g->ev2, g->ev3));
+  g->trace_n = 0;
+  *hs = h.st;
+  if (flow) *flow = h.flow;
+  return (wbpr_status)h.err;
+}
+
 wbpr_status run(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch_ms = nullptr) {
+  if (rc.mode != kModeFresh && use_resident(g, rc)) {
+    bool fits = false;
+    const wbpr_status st = run_resident(g, rc, hs, launch_ms, nullptr, &fits);
+    if (st || fits) return st;
+  }
   return g->layout == WBPR_LAYOUT_RCSR ? run_kernel<TopoR>(g, rc, hs, launch_ms)
                                        : run_kernel<TopoB>(g, rc, hs, launch_ms);
 }
@@ -1833,6 +1906,9 @@ wbpr_status make_cfg(wbpr_graph* g, int s, int t, wbpr_algo algo, const wbpr_tun
   const double ms = tu->max_ms > 0 ? tu->max_ms : 120000.0;
   rc->budget_ns = (unsigned long long)(ms * 1e6);
   rc->bfs_excl = -1;
+  rc->resident = !tu->tile && !tu->block && !tu->heavy_degree && !tu->blocks_per_sm && !tu->grid_blocks && !tu->trace &&
+                 alpha == kDefaultGrAlpha && !tu->gr_rounds && !tu->gr_stall && !tu->gr_plateau && !tu->bfs_alpha &&
+                 !tu->barrier_timeout_ns && !tu->greedy;
   return WBPR_OK;
 }
 
@@ -2120,20 +2196,27 @@ wbpr_status wbpr_solve(wbpr_graph* g, int32_t s, int32_t t, wbpr_algo algo, cons
   bool matched = false;
   if (rc.matching && (st = match_detect(g, s, t, &matched))) return st;
   CK(cudaEventRecord(g->ev0, g->stream));
-  if (g->layout == WBPR_LAYOUT_RCSR) {
-    if (g->m) reset_rcsr<<<g->sms * 8, 256, 0, g->stream>>>(g->farc, g->fcb, g->fcap, g->m);
-  } else {
-    restore_bcsr(g);
-  }
-  CK(cudaGetLastError());
   Stats hs;
   float launch_ms = 0;
-  st = matched ? run_match(g, rc, &hs, &launch_ms) : run(g, rc, &hs, &launch_ms);
-  CK(cudaEventRecord(g->ev1, g->stream));
+  int et = 0;
+  bool done = false;  // by the resident solver, which starts from the capacities itself
+  if (!matched && use_resident(g, rc)) {
+    st = run_resident(g, rc, &hs, &launch_ms, &et, &done);
+    if (done) CK(cudaEventRecord(g->ev1, g->stream));
+  }
+  if (!done) {
+    if (g->layout == WBPR_LAYOUT_RCSR) {
+      if (g->m) reset_rcsr<<<g->sms * 8, 256, 0, g->stream>>>(g->farc, g->fcb, g->fcap, g->m);
+    } else {
+      restore_bcsr(g);
+    }
+    CK(cudaGetLastError());
+    st = matched ? run_match(g, rc, &hs, &launch_ms) : run(g, rc, &hs, &launch_ms);
+    CK(cudaEventRecord(g->ev1, g->stream));
+  }
   CK(cudaEventSynchronize(g->ev1));
   if (st) return st;
-  int et = 0;
-  CK(cudaMemcpy(&et, g->e + t, 4, cudaMemcpyDeviceToHost));
+  if (!done) CK(cudaMemcpy(&et, g->e + t, 4, cudaMemcpyDeviceToHost));
   if (out) {
     std::memset(out, 0, sizeof(*out));
     out->flow = et;

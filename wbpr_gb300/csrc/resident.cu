@@ -1,0 +1,713 @@
+// Resident solver: push-relabel with the residual graph in shared memory.
+//
+// Small graphs are bound by latency, not by bytes: the persistent kernel
+// (pr_kernel.cuh) spends 10-20 us on a round or a BFS level of a graph of a
+// few thousand vertices, nearly all of it chains of dependent L2 accesses and
+// the grid barrier.  Here the whole residual graph sits in the shared memory
+// of one block, or of a cluster of 16 (distributed shared memory, the
+// hardware's cluster barrier), from its first load to the write-back: 8 bytes
+// an arc and 14 a vertex.  The vertices are split over the blocks in order,
+// by weight; a block owns its vertices' labels, excess and rows, and reaches
+// its neighbours' with remote loads and fire-and-forget remote reductions.
+// There are no queues: each step, every warp looks over the state of the
+// vertices it owns, which costs one shared-memory load a vertex and needs no
+// returning atomic.  A step pushes and relabels in one pass (discharge()), so
+// a round has one barrier instead of two.
+//
+// Measured on GB300, solve time before (persistent kernel) and now:
+//   GENRMF 4x5 (80 vertices, one block)            1.00 -> 0.13 ms
+//   GENRMF 8x16 (1,024 vertices, one block), RCSR  7.69 -> 0.69 ms
+//   layered 11x37 (409 vertices, one block), RCSR  1.91 -> 0.16 ms
+//   GENRMF 16x40 (10,240 vertices, cluster)        33.8 -> 3.74 ms
+//   layered 32x256 (8,194 vertices, cluster)       2.96 -> 0.53 ms
+//   R-MAT scale 13 (221k residual arcs, cluster)   0.70 -> 0.47 ms
+// A round takes 1.0-1.7 us in one block and about 2.2 us in the cluster, a BFS
+// level 0.6-0.8 us in one block; what bounds it now is the length of one
+// warp's instruction chain through discharge() (about 1,000 cycles) and, in
+// the cluster, the block that holds most of the active vertices.
+//
+// Blocks of 1,024 threads: with 512, a warp looks after twice the vertices one
+// after the other (GENRMF 8x16 0.89 against 0.67 ms).  A cluster is always 16
+// blocks: the least number that fits is slower (GENRMF 16x40 on 8: 4.9 ms,
+// layered 32x256 on 4: 0.85 ms), and a graph that fits one block is slower on
+// 16 (GENRMF 8x16: 0.80 ms).
+#include "resident.h"
+
+#include <cstddef>
+#include <mutex>
+
+namespace wbpr_dev {
+namespace {
+
+#ifndef WBPR_RES_THREADS
+#define WBPR_RES_THREADS 1024
+#endif
+constexpr int kResThreads = WBPR_RES_THREADS;
+
+// BFS levels a block runs between two cluster barriers (the search is
+// label-correcting).  GENRMF 16x40: 1 level 4.88, 8 3.76, 32 4.0-5.5 ms;
+// layered 32x256 0.85, 0.53, 0.5-0.8 ms.
+constexpr int kResBfsLevels = 8;
+// Global relabel once the rounds since the last one took this many sixteenths
+// of its time, and at least 8 rounds.  GENRMF 16x40 at 4, 8, 16: 9.2, 6.0,
+// 3.8 ms; the small graphs gain 0-10% from 8 to 16.
+constexpr int kResGrShare = 16;
+
+struct ResCtl {
+  int bnd[kResMaxCluster + 1];    // first vertex of every block of the cluster
+  int abase[kResMaxCluster + 1];  // its first residual arc
+  int busy[2];                    // number of the last barrier before which some block had work, by parity
+  int stop;                       // number of the barrier after which every block stops: budget exhausted
+  int gr;                         // number of the barrier after which every block relabels globally
+  unsigned long long sum[8];      // counters
+};
+
+__device__ __forceinline__ unsigned sm_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned cl_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned cl_size() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned cl_map(unsigned a, unsigned rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+
+// Shared memory of a block of the cluster (CL) or of this block.  at() gives
+// the address of the memory of block `rank`; every block lays it out alike.
+template <bool CL>
+struct Sh {
+  static __device__ __forceinline__ unsigned at(unsigned a0, unsigned rank) { return CL ? cl_map(a0, rank) : a0; }
+  static __device__ __forceinline__ int ld(unsigned a) {
+    int v;
+    if (CL) asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a));
+    else asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+  }
+  static __device__ __forceinline__ void st(unsigned a, int v) {
+    if (CL) asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+    else asm volatile("st.shared.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+  }
+  static __device__ __forceinline__ void st16(unsigned a, unsigned v) {
+    if (CL) asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
+    else asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
+  }
+  static __device__ __forceinline__ void add(unsigned a, int v) {
+    if (CL) asm volatile("red.relaxed.cluster.shared::cluster.add.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+    else asm volatile("red.relaxed.cta.shared.add.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+  }
+  static __device__ __forceinline__ void add64(unsigned a, unsigned long long v) {
+    if (CL) asm volatile("red.relaxed.cluster.shared::cluster.add.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+    else asm volatile("red.relaxed.cta.shared.add.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+  }
+  static __device__ __forceinline__ void min(unsigned a, int v) {
+    if (CL) asm volatile("red.relaxed.cluster.shared::cluster.min.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+    else asm volatile("red.relaxed.cta.shared.min.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+  }
+  static __device__ __forceinline__ void sync() {
+    if (CL) {
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else {
+      __syncthreads();
+    }
+  }
+};
+
+// The layout of one block's memory and its share of the graph.  The vertices
+// are dealt to the groups of 32 slots (a warp looks after a group) in turn, and
+// within a group to its four runs of 8 slots in turn: neighbours in vertex
+// order, which tend to be active together, fall to different warps, and the
+// few vertices of a small graph to as many warps and tiles as there are.
+struct Part {
+  ResCtl* c;
+  int2* rec;               // {residual, head (block << 12 | slot) | twin arc << 16}
+  int2* ve;                // {label, excess} by slot
+  unsigned* row;           // first arc | arcs << 16, by slot
+  unsigned short* ex;      // label a vertex was last expanded with in the running BFS, by slot
+  unsigned a0, a_rec, a_ve;  // shared-memory addresses: of the block's memory, of rec, of ve
+  int cs, rank;
+  unsigned a_row, a_ex;    // of row and ex
+  bool big;                // some row of this block is longer than a tile should walk
+  int groups;              // of 32 slots, the same in every block
+  int nv, na;              // vertices and arcs of this block
+  int n;                   // of the instance
+  int sv, tv;              // s and t as (block << 12 | slot), -1 for none
+  int sl, tl;              // s and t among this block's slots, or -1
+  __device__ __forceinline__ int slot(int j) const {
+    const int q = j / groups;
+    return (j - q * groups) * 32 + (q & 3) * 8 + (q >> 2);
+  }
+};
+
+struct Count {  // of one thread
+  unsigned scanned = 0, bfs = 0, pushes = 0, relabels = 0, visits = 0;
+};
+
+// Row offset of vertex v (0..n) in combined arc numbering.
+__device__ __forceinline__ int row_at(const ResInstance& in, int v) {
+  return in.row ? __ldg(in.row + in.vbase + v) : __ldg(in.frow + v) + __ldg(in.rrow + v);
+}
+
+// First vertex of block k: a 32-way search by one warp over the monotone
+// weight of the vertices before it.
+__device__ __forceinline__ int boundary(const ResInstance& in, int row0, long long total, int k, int cs) {
+  const int lane = threadIdx.x & 31;
+  const long long target = total * k / cs;
+  int lo = 0, hi = in.n;
+  while (lo < hi) {
+    const int step = (hi - lo + 31) >> 5;
+    const int x = lo + lane * step;
+    bool below = false;
+    if (x < hi) below = (long long)kResVertexBytes * x + (long long)kResArcBytes * (row_at(in, x) - row0) < target;
+    const int c = __popc(__ballot_sync(0xffffffffu, below));  // the predicate is monotone
+    if (c == 0) break;
+    const int nlo = lo + (c - 1) * step + 1;
+    hi = min(hi, lo + c * step);
+    lo = nlo;
+  }
+  return lo;
+}
+
+__device__ __forceinline__ int owner_of(const ResCtl* c, int cs, int v) {
+  int lo = 0, hi = cs;  // the last block whose first vertex is <= v
+  while (hi - lo > 1) {
+    const int m = (lo + hi) >> 1;
+    if (c->bnd[m] <= v) lo = m;
+    else hi = m;
+  }
+  return lo;
+}
+
+// Splits the instance over the cluster and lays out the memory; false when a
+// block's share does not fit (all blocks agree).
+template <bool CL>
+__device__ bool setup(const ResInstance& in, int smem_bytes, char* sm, Part& P) {
+  ResCtl* c = (ResCtl*)sm;
+  P.c = c;
+  P.cs = CL ? (int)cl_size() : 1;
+  P.rank = CL ? (int)cl_rank() : 0;
+  P.n = in.n;
+  const int row0 = row_at(in, 0);
+  const int rown = row_at(in, in.n);
+  const long long total = (long long)kResVertexBytes * in.n + (long long)kResArcBytes * (rown - row0);
+  const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int k = wid; k <= P.cs; k += nw) {
+    const int v = k == 0 ? 0 : (k == P.cs ? in.n : boundary(in, row0, total, k, P.cs));
+    if ((threadIdx.x & 31) == 0) {
+      c->bnd[k] = v;
+      c->abase[k] = row_at(in, v);
+    }
+  }
+  if (threadIdx.x < 8) c->sum[threadIdx.x] = 0;
+  if (threadIdx.x == 0) c->busy[0] = c->busy[1] = c->stop = c->gr = 0;
+  __syncthreads();
+  int nvmax = 0, namax = 0;
+  for (int k = 0; k < P.cs; ++k) {
+    nvmax = max(nvmax, c->bnd[k + 1] - c->bnd[k]);
+    namax = max(namax, c->abase[k + 1] - c->abase[k]);
+  }
+  P.groups = max((int)blockDim.x >> 5, (nvmax + 31) >> 5);
+  const int slots = 32 * P.groups;
+  char* q = sm + ((sizeof(ResCtl) + 15) & ~15u);
+  P.rec = (int2*)q;
+  q += 8 * (size_t)namax;
+  P.ve = (int2*)q;
+  q += 8 * (size_t)slots;
+  P.row = (unsigned*)q;
+  q += 4 * (size_t)slots;
+  P.ex = (unsigned short*)q;
+  q += 2 * (size_t)slots;
+  if (q > sm + smem_bytes || slots > kResMaxVertices || namax > kResMaxArcs) return false;
+  P.a0 = sm_addr(sm);
+  P.a_rec = sm_addr(P.rec) - P.a0;
+  P.a_ve = sm_addr(P.ve) - P.a0;
+  P.a_row = sm_addr(P.row);
+  P.a_ex = sm_addr(P.ex);
+  P.nv = c->bnd[P.rank + 1] - c->bnd[P.rank];
+  P.na = c->abase[P.rank + 1] - c->abase[P.rank];
+  P.sv = P.tv = P.sl = P.tl = -1;
+  if (in.s >= 0) {
+    const int o = owner_of(c, P.cs, in.s), l = P.slot(in.s - c->bnd[o]);
+    P.sv = o << 12 | l;
+    if (o == P.rank) P.sl = l;
+  }
+  {
+    const int o = owner_of(c, P.cs, in.t), l = P.slot(in.t - c->bnd[o]);
+    P.tv = o << 12 | l;
+    if (o == P.rank) P.tl = l;
+  }
+  return true;
+}
+
+// Rows longer than this are walked by a whole warp.
+template <int W>
+__host__ __device__ constexpr unsigned big_row() { return W == 32 ? 0xffffffffu : W * 16u; }
+
+// Reads this block's rows (residuals from the capacities in a fresh solve).
+template <int W, bool CL>
+__device__ void load(const ResInstance& in, Part& P) {
+  const ResCtl* c = P.c;
+  const int v0 = c->bnd[P.rank], a0 = c->abase[P.rank];
+  const bool fresh = in.mode == kModeFresh;
+  bool big = false;
+  for (int i = threadIdx.x; i < 32 * P.groups; i += blockDim.x) {
+    const int k = P.slot(i);
+    P.ve[k] = make_int2(P.n, 0);
+    P.row[k] = 0;
+    P.ex[k] = 0;
+    if (i >= P.nv) continue;
+    const int b = row_at(in, v0 + i) - a0, e = row_at(in, v0 + i + 1) - a0;
+    P.row[k] = (unsigned)b | (unsigned)(e - b) << 16;
+    big |= (unsigned)(e - b) > big_row<W>();
+    if (in.mode == kModeState) P.ve[k].y = __ldcg(in.e + in.vbase + v0 + i);
+  }
+  P.big = __syncthreads_or(big);
+  if (in.row) {
+#pragma unroll 4
+    for (int a = threadIdx.x; a < P.na; a += blockDim.x) {
+      const int2 r = __ldcg(in.arc + a0 + a), x = __ldg(in.arx + a0 + a);
+      const int d = r.x - in.vbase, o = owner_of(c, P.cs, d);
+      P.rec[a] = make_int2(fresh ? x.y : r.y, (int)((unsigned)(o << 12 | P.slot(d - c->bnd[o])) | (unsigned)(x.x - c->abase[o]) << 16));
+    }
+    Sh<CL>::sync();
+    return;
+  }
+  Sh<CL>::sync();  // every block's memory may be written from here on
+  const int sub = threadIdx.x & 7, tile = threadIdx.x >> 3, nt = blockDim.x >> 3;
+  for (int i = tile; i < P.nv; i += nt) {
+    const int v = v0 + i;
+    const int fb = __ldg(in.frow + v), fe = __ldg(in.frow + v + 1), rb = __ldg(in.rrow + v), re = __ldg(in.rrow + v + 1);
+    for (int f = fb + sub; f < fe; f += 8) {
+      const int2 r = __ldcg(in.farc + f);
+      const int o = owner_of(c, P.cs, r.x);
+      int2* q = P.rec + (f + rb - a0);
+      q->x = fresh ? __ldg(in.fcap + f) : r.y;
+      *(unsigned short*)&q->y = (unsigned short)(o << 12 | P.slot(r.x - c->bnd[o]));  // its twin is written below
+    }
+    for (int k = rb + sub; k < re; k += 8) {
+      const int2 r = __ldg(in.rarc + k);  // {tail, forward arc}
+      const int o = owner_of(c, P.cs, r.x);
+      const int here = fe + k - a0, tw = r.y + __ldg(in.rrow + r.x) - c->abase[o];
+      P.rec[here] = make_int2(fresh ? 0 : __ldcg(in.fcb + r.y), (int)((unsigned)(o << 12 | P.slot(r.x - c->bnd[o])) | (unsigned)tw << 16));
+      Sh<CL>::st16(Sh<CL>::at(P.a0, o) + P.a_rec + 8 * tw + 6, (unsigned)here);
+    }
+  }
+  Sh<CL>::sync();
+}
+
+__device__ void write_back(const ResInstance& in, const Part& P) {
+  const ResCtl* c = P.c;
+  const int v0 = c->bnd[P.rank], a0 = c->abase[P.rank];
+  for (int i = threadIdx.x; i < P.nv; i += blockDim.x) {
+    const int2 x = P.ve[P.slot(i)];
+    in.lab[in.vbase + v0 + i] = x.x;
+    if (in.mode != kModeBfsOnly) in.e[in.vbase + v0 + i] = x.y;
+  }
+  if (in.mode == kModeBfsOnly) return;
+  if (in.row) {
+    for (int a = threadIdx.x; a < P.na; a += blockDim.x) in.arc[a0 + a].y = P.rec[a].x;
+    return;
+  }
+  const int sub = threadIdx.x & 7, tile = threadIdx.x >> 3, nt = blockDim.x >> 3;
+  for (int i = tile; i < P.nv; i += nt) {
+    const int v = v0 + i;
+    const int fb = __ldg(in.frow + v), fe = __ldg(in.frow + v + 1), rb = __ldg(in.rrow + v);
+    for (int f = fb + sub; f < fe; f += 8) {
+      const int cf = P.rec[f + rb - a0].x;
+      in.farc[f].y = cf;
+      in.fcb[f] = __ldg(in.fcap + f) - cf;
+    }
+  }
+}
+
+__device__ __forceinline__ int2 lds64(unsigned a) {
+  int2 v;
+  asm volatile("ld.shared.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ unsigned lds32(unsigned a) {
+  unsigned v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ unsigned lds16(unsigned a) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+  return v;
+}
+
+// Whether any block of the cluster had work since its last call; every call
+// is a barrier of the cluster.  `seq` numbers the calls: a warp with work
+// posts the number to every block, so nothing has to be cleared.  There are
+// two words, because a fast block may post the next number before a slow one
+// has read this one (but not the number after it).
+template <bool CL>
+__device__ __forceinline__ bool any_work(const Part& P, bool did, int& seq) {
+  ++seq;
+  if (!CL) return __syncthreads_or(did);
+  if (did && (int)(threadIdx.x & 31) < P.cs)  // uniform over the warp
+    Sh<CL>::st(Sh<CL>::at(P.a0, threadIdx.x & 31) + (unsigned)offsetof(ResCtl, busy) + 4 * (seq & 1), seq);
+  Sh<CL>::sync();
+  return *(volatile int*)&P.c->busy[seq & 1] == seq;
+}
+
+constexpr unsigned kFull = 0xffffffffu;
+
+// Expands the vertices in slots u (one per W-lane tile, -1 for none) of label
+// l: lowers the labels of the heads (DIR 0: over arcs whose twin has residual).
+template <int W, bool CL, int DIR>
+__device__ __forceinline__ void bfs_expand(const Part& P, int u, int l, Count& ct) {
+  const unsigned lane = threadIdx.x & (W - 1);
+  const unsigned row = u >= 0 ? lds32(P.a_row + 4 * u) : 0;
+  const unsigned deg = row >> 16, rec = P.a0 + P.a_rec + 8 * (row & 0xffff);
+  const int nl = l + 1;
+  for (unsigned k = lane; k < deg; k += W) {
+    const int2 r = lds64(rec + 8 * k);
+    if (DIR == 1 && r.x <= 0) continue;
+    const unsigned d = r.y & 0xffff, m = Sh<CL>::at(P.a0, d >> 12), al = m + P.a_ve + 8 * (d & 0xfff);
+    const int lv = Sh<CL>::ld(al);
+    const int cf = DIR == 0 ? Sh<CL>::ld(m + P.a_rec + 8 * ((unsigned)r.y >> 16)) : 1;
+    if (lv > nl && cf > 0 && (int)d != P.sv) Sh<CL>::min(al, nl);
+  }
+  if (lane == 0) ct.bfs += deg;
+}
+
+// Exact distances to (DIR 0) or from (DIR 1) t over residual arcs, s never
+// labelled, n where there is none: label-correcting, `bsub` levels inside a
+// block between two cluster barriers.  Returns the levels of the longest run.
+template <int W, bool CL, int DIR>
+__device__ int bfs_resident(const ResParams& p, Part& P, int& seq, Count& ct) {
+  for (int i = threadIdx.x; i < 32 * P.groups; i += blockDim.x) {
+    P.ve[i].x = i == P.tl ? 0 : P.n;
+    P.ex[i] = (unsigned short)min(P.n, 65535);
+  }
+  Sh<CL>::sync();
+  int levels = 0;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (;;) {
+    bool did = false;
+    for (int k = 0; k < p.bsub; ++k) {
+      bool now = false;
+      for (int g = wid; g < P.groups; g += nw) {
+        const int i = g * 32 + lane;
+        const int l = (int)lds32(P.a0 + P.a_ve + 8 * i);
+        const bool open = l < (int)lds16(P.a_ex + 2 * i);
+        unsigned mask = __ballot_sync(kFull, open);
+        if (!mask) continue;
+        now = true;
+        if (open) P.ex[i] = (unsigned short)l;
+        if (W < 32 && P.big) {
+          unsigned big = __ballot_sync(kFull, open && P.row[i] >> 16 > big_row<W>());
+          mask &= ~big;
+          for (; big; big &= big - 1) {
+            const int t = __ffs(big) - 1;
+            bfs_expand<32, CL, DIR>(P, g * 32 + t, __shfl_sync(kFull, l, t), ct);
+          }
+        }
+        while (mask) {  // the k-th lowest open one goes to tile k
+          unsigned m = mask;
+#pragma unroll
+          for (int j = 0; j < 32 / W; ++j) {
+            if (j < lane / W) m &= m - 1;
+            mask &= mask - 1;
+          }
+          const int t = m ? __ffs(m) - 1 : -1;
+          const int lt = __shfl_sync(kFull, l, t & 31);
+          bfs_expand<W, CL, DIR>(P, t < 0 ? -1 : g * 32 + t, lt, ct);
+        }
+      }
+      did |= now;
+      if (k + 1 < p.bsub && !__syncthreads_or(now)) break;
+    }
+    if (!any_work<CL>(P, did, seq)) return levels;
+    levels += p.bsub;
+  }
+}
+
+// Push and relabel the active vertices in slots u (one per W-lane tile, -1
+// for none; whole warps call it).  A vertex's own label is the one it had when
+// the step began; a head's label may be read before or after that head's
+// relabel of the step.  An arc is admissible when the head's label is lower.
+// Of the two ends of an arc at most one can push along it in a step, because
+// an end only ever raises its label, after its pushes.  The new label is at
+// most two above the old one, which keeps it valid against pushes of the same
+// step into u that this scan has not seen: they come from labels at most one
+// above u's.
+template <int W, bool CL>
+__device__ __forceinline__ void discharge(const Part& P, int u, Count& ct) {
+  const unsigned lane = threadIdx.x & (W - 1);
+  int2 le = make_int2(0, 0);
+  unsigned row = 0;
+  if (u >= 0) {
+    le = lds64(P.a0 + P.a_ve + 8 * u);  // one read by the tile's lanes together
+    row = lds32(P.a_row + 4 * u);
+  }
+  const unsigned deg = row >> 16, rec = P.a0 + P.a_rec + 8 * (row & 0xffff);
+  const int hu = le.x;
+  unsigned erem = (unsigned)le.y, k = 0;
+  int mn = kBig;
+  constexpr int Q = 2;
+  do {
+    int2 r[Q];
+    unsigned m[Q], room[Q], own = 0;
+    int hv[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const unsigned i = k + q * W + lane;
+      r[q] = make_int2(0, 0);
+      if (i < deg && erem > 0) r[q] = lds64(rec + 8 * i);
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      m[q] = Sh<CL>::at(P.a0, (r[q].y & 0xf000) >> 12);
+      hv[q] = kBig;
+      if (r[q].x > 0) hv[q] = Sh<CL>::ld(m[q] + P.a_ve + 8 * (r[q].y & 0xfff));
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      room[q] = hv[q] < hu ? (unsigned)r[q].x : 0u;
+      own = min(own + room[q], erem);
+    }
+    if (__any_sync(kFull, own > 0)) {
+      // the tile's excess goes to its admissible arcs lane by lane
+      unsigned incl = own;
+#pragma unroll
+      for (int d = 1; d < W; d <<= 1) {
+        const unsigned y = __shfl_up_sync(kFull, incl, d, W);
+        if ((int)lane >= d) incl = min(incl + y, erem);
+      }
+      unsigned before = __shfl_up_sync(kFull, incl, 1, W);
+      if (lane == 0) before = 0;
+      const unsigned total = __shfl_sync(kFull, incl, W - 1, W);
+      unsigned left = erem - before;  // what this lane's arcs may take
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int push = (int)min(room[q], left);
+        left -= push;
+        if (push > 0) {
+          Sh<false>::add(rec + 8 * (k + q * W + lane), -push);
+          Sh<CL>::add(m[q] + P.a_rec + 8 * ((unsigned)r[q].y >> 16), push);
+          Sh<CL>::add(m[q] + P.a_ve + 8 * (r[q].y & 0xfff) + 4, push);
+          ++ct.pushes;
+        }
+        if (r[q].x > push) mn = min(mn, hv[q]);
+      }
+      erem -= total;
+    } else {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) mn = min(mn, hv[q]);
+    }
+    k += W * Q;
+  } while (__any_sync(kFull, k < deg && erem > 0));
+  if (__any_sync(kFull, erem > 0)) {
+#pragma unroll
+    for (int d = W / 2; d > 0; d >>= 1) mn = min(mn, __shfl_xor_sync(kFull, mn, d, W));
+    if (lane == 0 && erem > 0) {
+      P.ve[u].x = min(max(min(mn, hu + 1), hu) + 1, P.n);
+      ++ct.relabels;
+    }
+  }
+  if (lane == 0 && u >= 0) {
+    ct.scanned += min(k, deg);
+    ++ct.visits;
+    if (le.y > (int)erem) Sh<false>::add(P.a0 + P.a_ve + 8 * u + 4, (int)erem - le.y);
+  }
+}
+
+// One push / relabel step of this block; whether it had an active vertex.
+template <int W, bool CL>
+__device__ __forceinline__ bool push_step(const Part& P, Count& ct) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  bool did = false;
+  for (int g = wid; g < P.groups; g += nw) {
+    const int i = g * 32 + lane;
+    const int2 le = lds64(P.a0 + P.a_ve + 8 * i);
+    const bool act = le.y > 0 && le.x < P.n && i != P.tl;  // s keeps label n
+    unsigned mask = __ballot_sync(kFull, act);
+    if (!mask) continue;
+    did = true;
+    if (W < 32 && P.big) {
+      unsigned big = __ballot_sync(kFull, act && P.row[i] >> 16 > big_row<W>());
+      mask &= ~big;
+      for (; big; big &= big - 1) discharge<32, CL>(P, g * 32 + __ffs(big) - 1, ct);
+    }
+    // a tile takes the active ones among its own W slots
+    unsigned mine = W == 32 ? mask : mask >> (lane & ~(W - 1)) & ((1u << (W & 31)) - 1u);
+    while (__any_sync(kFull, mine)) {
+      discharge<W, CL>(P, mine ? g * 32 + (lane & ~(W - 1)) + __ffs(mine) - 1 : -1, ct);
+      mine &= mine - 1;
+    }
+  }
+  return did;
+}
+
+template <int W, bool CL>
+__device__ void solve_resident(const ResParams& p, Part& P, ResOut* out) {
+  const ResInstance& in = p.in;
+  Count ct;
+  int seq = 0, grs = 0, rounds = 0, since = 0, err = 0, total_levels = 0;
+  long long gr_end = 0, gr_len = 0, gr_all = 0;
+  const long long clk0 = clock64();
+  const unsigned long long t0 = gtime();
+  const int lane = threadIdx.x & 31;
+  if (in.mode == kModeBfsOnly) {
+    if (in.dir == 0) bfs_resident<W, CL, 0>(p, P, seq, ct);
+    else bfs_resident<W, CL, 1>(p, P, seq, ct);
+  } else {
+    if (in.mode == kModeFresh && P.sl >= 0) {
+      // preflow: saturate every residual arc out of s
+      const unsigned row = P.row[P.sl];
+      for (int k = threadIdx.x; k < (int)(row >> 16); k += blockDim.x) {
+        const int a = (row & 0xffff) + k;
+        const int2 r = P.rec[a];
+        const unsigned d = r.y & 0xffff, m = Sh<CL>::at(P.a0, d >> 12);
+        if (r.x <= 0 || (int)d == P.sv) continue;
+        P.rec[a].x = 0;
+        Sh<CL>::add(m + P.a_rec + 8 * ((unsigned)r.y >> 16), r.x);
+        Sh<CL>::add(m + P.a_ve + 8 * (d & 0xfff) + 4, r.x);
+      }
+    }
+    Sh<CL>::sync();
+    bool need_gr = true;
+    for (;;) {
+      if (need_gr) {
+        const long long c0 = clock64();
+        total_levels += bfs_resident<W, CL, 0>(p, P, seq, ct);
+        gr_end = clock64();
+        gr_len = gr_end - c0;
+        gr_all += gr_len;
+        ++grs;
+        since = 0;
+      }
+      const bool did = push_step<W, CL>(P, ct);
+      // the first block decides, and posts the number of the barrier below
+      // (not a flag: a slow block may read the word only after a fast one has
+      // reached the next barrier)
+      if (P.rank == 0 && threadIdx.x < P.cs) {
+        const unsigned to = Sh<CL>::at(P.a0, threadIdx.x);
+        // the cycle counter first (cheaper to read; an SM does over half a cycle per ns)
+        const bool out_of_time = (unsigned long long)(clock64() - clk0) >= p.budget_ns >> 1 && time_past(t0, p.budget_ns);
+        if ((p.max_rounds > 0 && rounds >= p.max_rounds) || out_of_time)
+          Sh<CL>::st(to + (unsigned)offsetof(ResCtl, stop), seq + 1);
+        if (since >= 8 && (clock64() - gr_end) * 16 >= gr_len * p.grp) Sh<CL>::st(to + (unsigned)offsetof(ResCtl, gr), seq + 1);
+      }
+      // the labels are valid after every step, so no active vertex means a
+      // maximum preflow
+      if (!any_work<CL>(P, did, seq)) break;
+      if (*(volatile int*)&P.c->stop == seq) {
+        err = (int)WBPR_ERR_NO_CONVERGENCE;
+        break;
+      }
+      need_gr = *(volatile int*)&P.c->gr == seq;
+      ++rounds;
+      ++since;
+    }
+  }
+  write_back(in, P);
+  // counters: warps into the block's words, blocks into the first block's
+  if (in.mode != kModeBfsOnly) {
+    int str = 0;
+    for (int i = threadIdx.x; i < 32 * P.groups; i += blockDim.x)
+      str += i != P.sl && i != P.tl && P.ve[i].y > 0 && P.ve[i].x >= P.n;
+    unsigned long long v[6] = {ct.scanned, ct.bfs, ct.pushes, ct.relabels, ct.visits, (unsigned)str};
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(kFull, v[k], o);
+      if (lane == 0 && v[k]) Sh<CL>::add64(Sh<CL>::at(P.a0, 0) + (unsigned)offsetof(ResCtl, sum) + 8 * k, v[k]);
+    }
+    if (P.tl >= 0 && threadIdx.x == 0) out->flow = P.ve[P.tl].y;
+    Sh<CL>::sync();
+  }
+  if (P.rank == 0 && threadIdx.x == 0) {
+    Stats s{};
+    s.arcs_scanned = P.c->sum[0];
+    s.bfs_arcs = P.c->sum[1];
+    s.pushes = P.c->sum[2];
+    s.relabels = P.c->sum[3];
+    s.vertex_visits = P.c->sum[4];
+    s.stranded = (int)P.c->sum[5];
+    s.rounds = rounds;
+    s.grs = grs;
+    s.bfs_levels = total_levels;
+    const unsigned long long ns = gtime() - t0;
+    s.gr_ns = (unsigned long long)((double)ns * (double)gr_all / (double)(clock64() - clk0));
+    s.push_ns = s.round_ns = ns - s.gr_ns;
+    out->st = s;
+    out->err = err;
+  }
+}
+
+extern __shared__ __align__(16) char res_smem[];
+
+template <int W, bool CL>
+__global__ void __launch_bounds__(kResThreads) pr_resident(const __grid_constant__ ResParams p) {
+  Part P;
+  if (!setup<CL>(p.in, p.smem_bytes, res_smem, P)) {
+    if (P.rank == 0 && threadIdx.x == 0) p.out->err = kResNoFit;
+    return;
+  }
+  load<W, CL>(p.in, P);
+  solve_resident<W, CL>(p, P, p.out);
+}
+
+template <int W, bool CL>
+cudaError_t launch_one(const ResParams& p, int cluster, cudaStream_t st) {
+  static std::mutex mu;
+  static bool ready[64] = {false};
+  const void* fn = (const void*)pr_resident<W, CL>;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    if (dev >= 64 || !ready[dev]) {
+      if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem)) != cudaSuccess) return e;
+      if (CL && (e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
+      if (dev < 64) ready[dev] = true;
+    }
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(cluster);
+  cfg.blockDim = dim3(kResThreads);
+  cfg.dynamicSmemBytes = kResSmem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = CL ? 1 : 0;
+  void* args[] = {(void*)&p};
+  return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
+}  // namespace
+
+int resident_cluster(long long n, long long na) {
+  const long long w = kResVertexBytes * n + kResArcBytes * na;
+  // a block's share of a cluster may exceed the mean by one row
+  auto fits = [&](long long cs) {
+    return (cs == 1 ? w : w + w / 32) <= cs * (kResSmem - kResHeader) && n <= cs * kResMaxVertices && na <= cs * kResMaxArcs;
+  };
+  return fits(1) ? 1 : (fits(kResMaxCluster) ? kResMaxCluster : 0);
+}
+
+cudaError_t launch_resident(const ResParams& p0, int tile, int cluster, cudaStream_t st) {
+  ResParams p = p0;
+  p.smem_bytes = kResSmem;
+  // measured on GB300: see the head of this file
+  p.bsub = cluster == 1 ? 1 : kResBfsLevels;
+  p.grp = kResGrShare;
+  if (cluster == 1) return tile < 32 ? launch_one<8, false>(p, 1, st) : launch_one<32, false>(p, 1, st);
+  return tile < 32 ? launch_one<8, true>(p, cluster, st) : launch_one<32, true>(p, cluster, st);
+}
+
+}  // namespace wbpr_dev
