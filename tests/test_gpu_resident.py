@@ -1,5 +1,6 @@
 """The resident solver (the residual graph in the shared memory of one block
-or of a 16-block cluster) at the sizes where its split can go wrong, against
+or of a 16-block cluster) and the hybrid one (its vertices there, its arcs in
+global memory) at the sizes where their split can go wrong, against
 the oracle and against the persistent kernel (which any of its own knobs, such
 as `tile`, selects): exact flow, valid labels and the device certificate, both
 extreme minimum cuts, and the completed flow, on both layouts and algorithms.
@@ -42,6 +43,11 @@ CASES = {
     "long rows in a cluster": lambda: W.gen_rmat(13, 14, seed=5),
     "a row of several blocks' arcs": lambda: _star(29000, 6),  # fits no block: the persistent kernel takes it
     "a cluster nearly full": lambda: W.gen_layered(64, 480, 3, 6, 1, 1000, 7),
+    "hybrid": lambda: W.gen_layered(31, 641, 3, 6, 1, 1000, 8),
+    "hybrid, every vertex active at once": lambda: W.gen_layered(3, 30011, 3, 6, 1, 1000, 9),
+    "hybrid, rows in global memory": lambda: W.gen_grid(431, 419, 10),
+    "the largest hybrid": lambda: W.gen_layered(20, 14233, 3, 6, 1, 50, 11),  # 284,662 vertices of at most 284,672
+    "one more than the largest hybrid": lambda: W.gen_layered(5, 56935, 3, 6, 1, 50, 12),
     "a deep path over a cluster": lambda: W.Graph.from_arcs(9000, np.arange(8999), np.arange(1, 9000),
                                                             np.full(8999, 3), 0, 8999),
 }
@@ -51,8 +57,7 @@ CASES = {
 @pytest.mark.parametrize("layout", ["bcsr", "rcsr"])
 def test_resident_solver_agrees(name, layout):
     g = CASES[name]()
-    flow = oracle.dinic(g.n, g.off, g.dst, g.cap, g.s, g.t)
-    _, sink_ind, source_ind = oracle.mincut(g.n, g.off, g.dst, g.cap, g.s, g.t)
+    flow, sink_ind, source_ind = oracle.mincut(g.n, g.off, g.dst, g.cap, g.s, g.t)
     tail = np.repeat(np.arange(g.n), np.diff(g.off))
     inner = np.ones(g.n, bool)
     inner[[g.s, g.t]] = False

@@ -183,6 +183,8 @@ struct wbpr_graph {
   // resident solver: blocks of the cluster whose shared memory holds the
   // graph (0: none does), and what its launch reports
   int res_cluster = 0;
+  bool hybrid = false;       // else the hybrid solver takes it, with one record an arc
+  int4* hyb_rec = nullptr;
   ResOut* res_out = nullptr;
   int64_t bytes = 0;
   std::vector<void*> allocs;
@@ -1420,6 +1422,9 @@ wbpr_status create_impl(const wbpr_csr* in, wbpr_layout layout, wbpr_graph** out
   const int n = g->n;
   TRY(build_device(g, in));
   g->res_cluster = resident_cluster(g->n, g->total_deg);
+  g->hybrid = hybrid_takes(g->n, g->total_deg, g->n_medium + g->n_heavy);
+  // both could: see kResPreferUnits
+  if (g->res_cluster > 1 && g->hybrid && g->n + g->total_deg > kResPreferUnits) g->res_cluster = 0;
   int** vec[] = {&g->h, &g->e, &g->rl_min, &g->rl_left, &g->lq[0], &g->lq[1], &g->hq[0], &g->hq[1],
                  &g->esnap, &g->dmin0,
                  &g->qraw, &g->fr[0], &g->fr[1], &g->fr[2], &g->vlab};
@@ -1632,58 +1637,78 @@ wbpr_status run_kernel(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch
   return WBPR_OK;
 }
 
-bool use_resident(const wbpr_graph* g, const RunCfg& rc) { return rc.resident && !rc.term && g->res_cluster > 0; }
+bool use_resident(const wbpr_graph* g, const RunCfg& rc) {
+  return rc.resident && !rc.term && (g->res_cluster > 0 || g->hybrid);
+}
 
-// One launch of the resident solver.  *fits is cleared (and the handle's
-// cluster size raised, or set to 0) when a block's share of the graph is
-// larger than its shared memory; nothing has changed then.
+// One launch of the resident or the hybrid solver.  *fits is cleared when
+// neither can take the graph after all (a row too long for a block's share, a
+// device without such clusters); nothing has changed then.
 wbpr_status run_resident(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch_ms, int* flow, bool* fits) {
   *fits = true;
   if (!g->res_out) {
     wbpr_status st = dalloc(g, &g->res_out, 1);
     if (st) return st;
   }
-  ResParams p{};
-  p.in.n = g->n;
-  p.in.mode = rc.mode;
-  p.in.s = rc.mode == kModeBfsOnly ? rc.bfs_excl : rc.s;
-  p.in.t = rc.mode == kModeBfsOnly ? rc.bfs_root : rc.t;
-  p.in.dir = rc.bfs_dir;
+  ResInstance in{};
+  in.n = g->n;
+  in.mode = rc.mode;
+  in.s = rc.mode == kModeBfsOnly ? rc.bfs_excl : rc.s;
+  in.t = rc.mode == kModeBfsOnly ? rc.bfs_root : rc.t;
+  in.dir = rc.bfs_dir;
   if (g->layout == WBPR_LAYOUT_BCSR) {
-    p.in.row = g->row;
-    p.in.arc = g->arc;
-    p.in.arx = g->arx;
+    in.row = g->row;
+    in.arc = g->arc;
+    in.arx = g->arx;
   } else {
-    p.in.frow = g->frow;
-    p.in.farc = g->farc;
-    p.in.fcb = g->fcb;
-    p.in.fcap = g->fcap;
-    p.in.rrow = g->rrow;
-    p.in.rarc = g->rarc;
+    in.frow = g->frow;
+    in.farc = g->farc;
+    in.fcb = g->fcb;
+    in.fcap = g->fcap;
+    in.rrow = g->rrow;
+    in.rarc = g->rarc;
   }
-  p.in.lab = rc.lab ? rc.lab : g->h;
-  p.in.e = g->e;
-  p.out = g->res_out;
-  p.max_rounds = rc.max_rounds;
-  p.budget_ns = rc.budget_ns;
+  in.lab = rc.lab ? rc.lab : g->h;
+  in.e = g->e;
   ResOut h;
   for (;;) {
-    if (launch_ms) CK(cudaEventRecord(g->ev2, g->stream));
-    if (launch_resident(p, g->avg_deg < 20 ? 8 : 32, g->res_cluster, g->stream) != cudaSuccess) {
-      cudaGetLastError();  // no such cluster on this device: the persistent kernel takes the graph
-      g->res_cluster = 0;
+    if (g->res_cluster == 0 && !g->hybrid) {
       *fits = false;
       return WBPR_OK;
+    }
+    if (g->res_cluster == 0 && !g->hyb_rec) {
+      wbpr_status st = dalloc(g, &g->hyb_rec, 2 * (size_t)g->m);
+      if (st) return st;
+    }
+    if (launch_ms) CK(cudaEventRecord(g->ev2, g->stream));
+    cudaError_t e;
+    if (g->res_cluster) {
+      ResParams p{};
+      p.in = in;
+      p.out = g->res_out;
+      p.max_rounds = rc.max_rounds;
+      p.budget_ns = rc.budget_ns;
+      e = launch_resident(p, g->avg_deg < 20 ? 8 : 32, g->res_cluster, g->stream);
+    } else {
+      HybParams p{};
+      p.in = in;
+      p.out = g->res_out;
+      p.rec = g->hyb_rec;
+      p.max_rounds = rc.max_rounds;
+      p.budget_ns = rc.budget_ns;
+      e = launch_hybrid(p, g->stream);
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // no such cluster on this device: the persistent kernel takes the graph
+      g->res_cluster = 0;
+      g->hybrid = false;
+      continue;
     }
     if (launch_ms) CK(cudaEventRecord(g->ev3, g->stream));
     CK(cudaMemcpyAsync(&h, g->res_out, sizeof(h), cudaMemcpyDeviceToHost, g->stream));
     CK(cudaStreamSynchronize(g->stream));
     if (h.err != kResNoFit) break;
-    g->res_cluster = g->res_cluster < kResMaxCluster ? 2 * g->res_cluster : 0;
-    if (!g->res_cluster) {
-      *fits = false;
-      return WBPR_OK;
-    }
+    g->res_cluster = g->res_cluster < kResMaxCluster ? kResMaxCluster : 0;
   }
   if (rc.mode != kModeBfsOnly) g->full_reset = true;  // its pushes are not in the undo log
   if (launch_ms) CK(cudaEventElapsedTime(launch_ms, g->ev2, g->ev3));

@@ -31,18 +31,12 @@
 // blocks: the least number that fits is slower (GENRMF 16x40 on 8: 4.9 ms,
 // layered 32x256 on 4: 0.85 ms), and a graph that fits one block is slower on
 // 16 (GENRMF 8x16: 0.80 ms).
+#include "resident.cuh"
 #include "resident.h"
-
-#include <cstddef>
-#include <mutex>
 
 namespace wbpr_dev {
 namespace {
 
-#ifndef WBPR_RES_THREADS
-#define WBPR_RES_THREADS 1024
-#endif
-constexpr int kResThreads = WBPR_RES_THREADS;
 
 // BFS levels a block runs between two cluster barriers (the search is
 // label-correcting).  GENRMF 16x40: 1 level 4.88, 8 3.76, 32 4.0-5.5 ms;
@@ -52,73 +46,6 @@ constexpr int kResBfsLevels = 8;
 // of its time, and at least 8 rounds.  GENRMF 16x40 at 4, 8, 16: 9.2, 6.0,
 // 3.8 ms; the small graphs gain 0-10% from 8 to 16.
 constexpr int kResGrShare = 16;
-
-struct ResCtl {
-  int bnd[kResMaxCluster + 1];    // first vertex of every block of the cluster
-  int abase[kResMaxCluster + 1];  // its first residual arc
-  int busy[2];                    // number of the last barrier before which some block had work, by parity
-  int stop;                       // number of the barrier after which every block stops: budget exhausted
-  int gr;                         // number of the barrier after which every block relabels globally
-  unsigned long long sum[8];      // counters
-};
-
-__device__ __forceinline__ unsigned sm_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned cl_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ unsigned cl_size() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ unsigned cl_map(unsigned a, unsigned rank) {
-  unsigned r;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  return r;
-}
-
-// Shared memory of a block of the cluster (CL) or of this block.  at() gives
-// the address of the memory of block `rank`; every block lays it out alike.
-template <bool CL>
-struct Sh {
-  static __device__ __forceinline__ unsigned at(unsigned a0, unsigned rank) { return CL ? cl_map(a0, rank) : a0; }
-  static __device__ __forceinline__ int ld(unsigned a) {
-    int v;
-    if (CL) asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a));
-    else asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-  }
-  static __device__ __forceinline__ void st(unsigned a, int v) {
-    if (CL) asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-    else asm volatile("st.shared.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-  }
-  static __device__ __forceinline__ void st16(unsigned a, unsigned v) {
-    if (CL) asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
-    else asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
-  }
-  static __device__ __forceinline__ void add(unsigned a, int v) {
-    if (CL) asm volatile("red.relaxed.cluster.shared::cluster.add.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-    else asm volatile("red.relaxed.cta.shared.add.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-  }
-  static __device__ __forceinline__ void add64(unsigned a, unsigned long long v) {
-    if (CL) asm volatile("red.relaxed.cluster.shared::cluster.add.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
-    else asm volatile("red.relaxed.cta.shared.add.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
-  }
-  static __device__ __forceinline__ void min(unsigned a, int v) {
-    if (CL) asm volatile("red.relaxed.cluster.shared::cluster.min.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-    else asm volatile("red.relaxed.cta.shared.min.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-  }
-  static __device__ __forceinline__ void sync() {
-    if (CL) {
-      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    } else {
-      __syncthreads();
-    }
-  }
-};
 
 // The layout of one block's memory and its share of the graph.  The vertices
 // are dealt to the groups of 32 slots (a warp looks after a group) in turn, and
@@ -145,15 +72,6 @@ struct Part {
     return (j - q * groups) * 32 + (q & 3) * 8 + (q >> 2);
   }
 };
-
-struct Count {  // of one thread
-  unsigned scanned = 0, bfs = 0, pushes = 0, relabels = 0, visits = 0;
-};
-
-// Row offset of vertex v (0..n) in combined arc numbering.
-__device__ __forceinline__ int row_at(const ResInstance& in, int v) {
-  return in.row ? __ldg(in.row + in.vbase + v) : __ldg(in.frow + v) + __ldg(in.rrow + v);
-}
 
 // First vertex of block k: a 32-way search by one warp over the monotone
 // weight of the vertices before it.
@@ -327,39 +245,6 @@ __device__ void write_back(const ResInstance& in, const Part& P) {
   }
 }
 
-__device__ __forceinline__ int2 lds64(unsigned a) {
-  int2 v;
-  asm volatile("ld.shared.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ unsigned lds32(unsigned a) {
-  unsigned v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ unsigned lds16(unsigned a) {
-  unsigned short v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
-  return v;
-}
-
-// Whether any block of the cluster had work since its last call; every call
-// is a barrier of the cluster.  `seq` numbers the calls: a warp with work
-// posts the number to every block, so nothing has to be cleared.  There are
-// two words, because a fast block may post the next number before a slow one
-// has read this one (but not the number after it).
-template <bool CL>
-__device__ __forceinline__ bool any_work(const Part& P, bool did, int& seq) {
-  ++seq;
-  if (!CL) return __syncthreads_or(did);
-  if (did && (int)(threadIdx.x & 31) < P.cs)  // uniform over the warp
-    Sh<CL>::st(Sh<CL>::at(P.a0, threadIdx.x & 31) + (unsigned)offsetof(ResCtl, busy) + 4 * (seq & 1), seq);
-  Sh<CL>::sync();
-  return *(volatile int*)&P.c->busy[seq & 1] == seq;
-}
-
-constexpr unsigned kFull = 0xffffffffu;
-
 // Expands the vertices in slots u (one per W-lane tile, -1 for none) of label
 // l: lowers the labels of the heads (DIR 0: over arcs whose twin has residual).
 template <int W, bool CL, int DIR>
@@ -426,7 +311,7 @@ __device__ int bfs_resident(const ResParams& p, Part& P, int& seq, Count& ct) {
       did |= now;
       if (k + 1 < p.bsub && !__syncthreads_or(now)) break;
     }
-    if (!any_work<CL>(P, did, seq)) return levels;
+    if (!any_work<CL>(P.c, P.a0, P.cs, did, seq)) return levels;
     levels += p.bsub;
   }
 }
@@ -600,7 +485,7 @@ __device__ void solve_resident(const ResParams& p, Part& P, ResOut* out) {
       }
       // the labels are valid after every step, so no active vertex means a
       // maximum preflow
-      if (!any_work<CL>(P, did, seq)) break;
+      if (!any_work<CL>(P.c, P.a0, P.cs, did, seq)) break;
       if (*(volatile int*)&P.c->stop == seq) {
         err = (int)WBPR_ERR_NO_CONVERGENCE;
         break;
@@ -658,37 +543,6 @@ __global__ void __launch_bounds__(kResThreads) pr_resident(const __grid_constant
   solve_resident<W, CL>(p, P, p.out);
 }
 
-template <int W, bool CL>
-cudaError_t launch_one(const ResParams& p, int cluster, cudaStream_t st) {
-  static std::mutex mu;
-  static bool ready[64] = {false};
-  const void* fn = (const void*)pr_resident<W, CL>;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (dev >= 64 || !ready[dev]) {
-      if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem)) != cudaSuccess) return e;
-      if (CL && (e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
-      if (dev < 64) ready[dev] = true;
-    }
-  }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(cluster);
-  cfg.blockDim = dim3(kResThreads);
-  cfg.dynamicSmemBytes = kResSmem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = cluster;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = CL ? 1 : 0;
-  void* args[] = {(void*)&p};
-  return cudaLaunchKernelExC(&cfg, fn, args);
-}
-
 }  // namespace
 
 int resident_cluster(long long n, long long na) {
@@ -706,8 +560,8 @@ cudaError_t launch_resident(const ResParams& p0, int tile, int cluster, cudaStre
   // measured on GB300: see the head of this file
   p.bsub = cluster == 1 ? 1 : kResBfsLevels;
   p.grp = kResGrShare;
-  if (cluster == 1) return tile < 32 ? launch_one<8, false>(p, 1, st) : launch_one<32, false>(p, 1, st);
-  return tile < 32 ? launch_one<8, true>(p, cluster, st) : launch_one<32, true>(p, cluster, st);
+  if (cluster == 1) return tile < 32 ? launch_cluster<pr_resident<8, false>>(p, 1, st) : launch_cluster<pr_resident<32, false>>(p, 1, st);
+  return tile < 32 ? launch_cluster<pr_resident<8, true>>(p, cluster, st) : launch_cluster<pr_resident<32, true>>(p, cluster, st);
 }
 
 }  // namespace wbpr_dev

@@ -1,0 +1,158 @@
+// Device helpers shared by the solvers that keep a graph, or its vertices, in
+// the shared memory of one thread block or of one thread-block cluster.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <mutex>
+
+#include "resident.h"
+
+namespace wbpr_dev {
+namespace {
+
+constexpr int kResThreads = 1024;
+constexpr unsigned kFull = 0xffffffffu;
+
+struct ResCtl {
+  int bnd[kResMaxCluster + 1];    // first vertex of every block of the cluster
+  int abase[kResMaxCluster + 1];  // its first residual arc
+  int busy[2];                    // number of the last barrier before which some block had work, by parity
+  int stop;                       // number of the barrier after which every block stops: budget exhausted
+  int gr;                         // number of the barrier after which every block relabels globally
+  unsigned long long sum[8];      // counters
+};
+
+__device__ __forceinline__ unsigned sm_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned cl_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned cl_size() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned cl_map(unsigned a, unsigned rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+
+// Shared memory of a block of the cluster (CL) or of this block.  at() gives
+// the address of the memory of block `rank`; every block lays it out alike.
+template <bool CL>
+struct Sh {
+  static __device__ __forceinline__ unsigned at(unsigned a0, unsigned rank) { return CL ? cl_map(a0, rank) : a0; }
+  static __device__ __forceinline__ int ld(unsigned a) {
+    int v;
+    if (CL) asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a));
+    else asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+  }
+  static __device__ __forceinline__ void st(unsigned a, int v) {
+    if (CL) asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+    else asm volatile("st.shared.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+  }
+  static __device__ __forceinline__ void st16(unsigned a, unsigned v) {
+    if (CL) asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
+    else asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
+  }
+  static __device__ __forceinline__ void add(unsigned a, int v) {
+    if (CL) asm volatile("red.relaxed.cluster.shared::cluster.add.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+    else asm volatile("red.relaxed.cta.shared.add.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+  }
+  static __device__ __forceinline__ void add64(unsigned a, unsigned long long v) {
+    if (CL) asm volatile("red.relaxed.cluster.shared::cluster.add.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+    else asm volatile("red.relaxed.cta.shared.add.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+  }
+  static __device__ __forceinline__ void min(unsigned a, int v) {
+    if (CL) asm volatile("red.relaxed.cluster.shared::cluster.min.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+    else asm volatile("red.relaxed.cta.shared.min.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+  }
+  static __device__ __forceinline__ void sync() {
+    if (CL) {
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else {
+      __syncthreads();
+    }
+  }
+};
+
+__device__ __forceinline__ int2 lds64(unsigned a) {
+  int2 v;
+  asm volatile("ld.shared.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ unsigned lds32(unsigned a) {
+  unsigned v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ unsigned lds16(unsigned a) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+  return v;
+}
+
+// Whether any block of the cluster had work since its last call; every call
+// is a barrier of the cluster.  `seq` numbers the calls: a warp with work
+// posts the number to every block, so nothing has to be cleared.  There are
+// two words, because a fast block may post the next number before a slow one
+// has read this one (but not the number after it).
+template <bool CL>
+__device__ __forceinline__ bool any_work(ResCtl* c, unsigned a0, int cs, bool did, int& seq) {
+  ++seq;
+  if (!CL) return __syncthreads_or(did);
+  if (did && (int)(threadIdx.x & 31) < cs)  // uniform over the warp
+    Sh<CL>::st(Sh<CL>::at(a0, threadIdx.x & 31) + (unsigned)offsetof(ResCtl, busy) + 4 * (seq & 1), seq);
+  Sh<CL>::sync();
+  return *(volatile int*)&c->busy[seq & 1] == seq;
+}
+
+struct Count {  // of one thread
+  unsigned scanned = 0, bfs = 0, pushes = 0, relabels = 0, visits = 0;
+};
+
+// Row offset of vertex v (0..n) in combined arc numbering.
+__device__ __forceinline__ int row_at(const ResInstance& in, int v) {
+  return in.row ? __ldg(in.row + in.vbase + v) : __ldg(in.frow + v) + __ldg(in.rrow + v);
+}
+
+// Launches one cluster of `blocks` blocks (1: no cluster) with the whole shared
+// memory of an SM each.
+template <auto Fn, class Prm>
+cudaError_t launch_cluster(const Prm& p, int blocks, cudaStream_t st, int clusters = 1) {
+  static std::mutex mu;
+  static bool ready[64] = {false};  // of this kernel, by device
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    if (dev >= 64 || !ready[dev]) {
+      if ((e = cudaFuncSetAttribute((const void*)Fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem)) != cudaSuccess) return e;
+      if (blocks > 1 && (e = cudaFuncSetAttribute((const void*)Fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
+      if (dev < 64) ready[dev] = true;
+    }
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks * clusters);
+  cfg.blockDim = dim3(kResThreads);
+  cfg.dynamicSmemBytes = kResSmem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = blocks;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = blocks > 1 ? 1 : 0;
+  void* args[] = {(void*)&p};
+  return cudaLaunchKernelExC(&cfg, (const void*)Fn, args);
+}
+
+}  // namespace
+}  // namespace wbpr_dev

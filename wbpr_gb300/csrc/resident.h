@@ -57,6 +57,40 @@ struct ResParams {
   int grp;    // global relabel when the rounds since the last one took grp / 16 x its time
 };
 
+// The hybrid solver: the vertices in the shared memory of a 16-block cluster,
+// the arcs as 16-byte records in global memory.
+constexpr int kHybVertexBytes = 12;     // label, excess, expanded label
+constexpr int kHybRowBytes = 8;         // the row, where there is room for it
+constexpr int kHybListBytes = 32 * 512;  // 256 slots a warp
+constexpr int kHybMaxVertices = kResMaxCluster * ((kResSmem - kResHeader - kHybListBytes) / kHybVertexBytes / 128 * 128);
+
+struct HybParams {
+  ResInstance in;
+  ResOut* out;
+  int4* rec;  // one record a residual arc: (hybrid.cu)
+  long long max_rounds;
+  unsigned long long budget_ns;
+  int bsub;
+  int grp;
+};
+
+// Whether the hybrid solver should take a graph: n vertices, na residual arcs,
+// `longer` of its rows longer than kLightDeg arcs.
+// (Sparse graphs, whose many short rounds and levels are what a solve waits
+// for: on R-MAT scale 13 one warp's walk of a long row makes it 1.0 ms against
+// 0.47 resident, and a large power-law graph has a dozen rounds that need all
+// SMs' bandwidth.)
+inline bool hybrid_takes(long long n, long long na, long long longer) {
+  return n <= kHybMaxVertices && na < 20 * n && longer <= 2 + n / 256;
+}
+cudaError_t launch_hybrid(const HybParams& p, cudaStream_t st);
+
+// Above this many vertices and residual arcs a graph that both could take goes
+// to the hybrid solver: its vertices are dealt to the blocks one by one, the
+// resident solver's in runs.  GENRMF 16x40 (107k units) 3.9 ms resident, 4.7
+// hybrid; layered 32x256 (80k) 0.52, 0.49; layered 64x512 (324k) 2.03, 1.10.
+constexpr long long kResPreferUnits = 1 << 17;
+
 // Cluster size for a graph of n vertices and na residual arcs: the smallest
 // power of two whose shared memory holds it, or 0.
 int resident_cluster(long long n, long long na);
