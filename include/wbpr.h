@@ -121,8 +121,9 @@ typedef struct wbpr_tuning {
                          /* the general solver                                    */
   int32_t pad2;
   int64_t batch_cluster; /* batches: instances of at least this many units (n +   */
-                         /* residual arcs) run on 8-block thread-block clusters, */
-                         /* the rest one block each (0 = 3 x 2^17, -1 = none)     */
+                         /* residual arcs) run on thread-block clusters, the rest */
+                         /* one block each; 0 = every instance on the fewest      */
+                         /* blocks that end before the batch can, -1 = none       */
 } wbpr_tuning;
 
 typedef struct wbpr_result {

@@ -1,14 +1,17 @@
 // Batched solver: many independent, uneven max-flow instances in one launch.
 //
 // All instances live in one concatenated BCSR16 graph (global vertex and arc
-// ids).  Each thread block claims a whole instance from a work list sorted by
-// size (largest first) and solves it alone: preflow, then global relabels
-// (block-level BFS from the sink) and synchronous push/relabel rounds with
-// __syncthreads as the only barrier, each instance scheduling its own global
-// relabels by its own work and round counts.  Blocks never wait for each
-// other, so the launch needs no grid barrier.  Per-instance device
-// timestamps give the latency distribution.  The launch (and the memset of
-// its work counter) is captured once into a CUDA graph and replayed.
+// ids).  Most of them go to the resident and hybrid solvers (resident.cu,
+// hybrid.cu; see capture() below).  This file's own kernel takes the rest, and
+// all of them when one of its knobs is set: each thread block claims a whole
+// instance from a work list sorted by size (largest first) and solves it
+// alone: preflow, then global relabels (block-level BFS from the sink) and
+// synchronous push/relabel rounds with __syncthreads as the only barrier, each
+// instance scheduling its own global relabels by its own work and round
+// counts.  Blocks never wait for each other, so the launch needs no grid
+// barrier.  Per-instance device timestamps give the latency distribution.  The
+// launches (and the memset of their work counters) are captured once into a
+// CUDA graph and replayed.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -21,17 +24,16 @@
 
 #include "devmem.h"
 #include "pr_kernel.cuh"
+#include "resident.h"
 #include "wbpr_internal.h"
 
 using namespace wbpr_dev;
 
-struct BatchInst {
-  int vbase;  // first global vertex id
-  int n;      // vertices
-  int s, t;   // global ids
-};
+using BatchInst = ResInst;
 
 struct wbpr_batch {
+  static constexpr int kLaunches = 8;          // concurrent launches of a batch, at most
+  static constexpr int kSides = kLaunches - 1;  // the last one is on `stream`
   int device = 0, sms = 0, count = 0;
   int64_t total_n = 0, total_arcs = 0, bytes = 0;
   cudaStream_t stream = nullptr;
@@ -52,11 +54,18 @@ struct wbpr_batch {
   long long* flows = nullptr;
   unsigned long long* inst_ns = nullptr;
   int* inst_rounds = nullptr;
-  int* next = nullptr;  // work-list cursors: one-block instances, cluster instances
-  int* next_big = nullptr;
-  std::vector<int64_t> size_sorted;  // instance sizes (n + residual arcs), largest first
-  cudaStream_t side = nullptr;       // second branch of the captured launch
-  cudaEvent_t fork = nullptr, join = nullptr;
+  int* next = nullptr;  // work-list cursors, one a launch of the captured graph
+  struct Shape {
+    int64_t n, arcs;
+    int64_t longer;  // rows of more than kLightDeg arcs
+    int64_t units() const { return n + arcs; }
+  };
+  std::vector<Shape> shape;          // by instance
+  std::vector<int32_t> host_order;   // instance ids, largest first
+  cudaStream_t side[kSides] = {};    // the other branches of the captured launch
+  cudaEvent_t fork = nullptr, join[kSides] = {};
+  int4* rec = nullptr;               // the hybrid solver's arc records
+  int64_t rec_count = 0;
   std::vector<void*> allocs;
   // captured launch
   cudaGraphExec_t exec = nullptr;
@@ -64,7 +73,9 @@ struct wbpr_batch {
   double cap_alpha = 0;
   int cap_grr = 0;
   int64_t cap_cluster = -2;
-  int cap_nbig = 0;
+  bool cap_mixed = false;
+  long long cap_rounds = 0;
+  double cap_ms = 0;
   std::vector<long long> host_flows;
 };
 
@@ -370,8 +381,10 @@ void batch_release(wbpr_batch* b) {
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->fork) cudaEventDestroy(b->fork);
-  if (b->join) cudaEventDestroy(b->join);
-  if (b->side) cudaStreamDestroy(b->side);
+  for (int k = 0; k < wbpr_batch::kSides; ++k) {
+    if (b->join[k]) cudaEventDestroy(b->join[k]);
+    if (b->side[k]) cudaStreamDestroy(b->side[k]);
+  }
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
 }
@@ -399,31 +412,112 @@ const void* kernel_for(int tile, bool cluster) {
   return nullptr;
 }
 
-// Capture the batch launch as a CUDA graph: the instances of at least
-// `cluster_units` units (a prefix of the largest-first order) on a second
-// branch, one 8-block cluster each, claimed from their own work list by as
-// many clusters as fit at once; the rest one block each, taking the SMs the
-// clusters leave and then the ones they give back as their list drains.  The
-// largest instances set the batch's makespan (one of 64k vertices takes
-// 440 ms on a block, ~2,800 rounds; 130 ms on a cluster), so they are the
-// ones that get more threads.  Measured on 4,096 uneven instances (half
-// GENRMF, a and b log-uniform in [4, 32] x [4, 64], half layered networks)
-// (block 512, tile 8): 434 ms with no clusters; from 2^19, 3 x 2^17, 2^18
-// and 3 x 2^16 units 357, 269, 319 and 368 ms (p99 per instance 180, 150,
-// 114 and 94 ms); half the clusters instead of all of them: 352, 273, 363
-// and 476 ms.
+// Cluster sizes of the hybrid solver, largest first, and about how long it
+// takes on each, in ns a unit (n + residual arcs) of a GENRMF, the family with
+// the most rounds.  Measured on GB300 alone: GENRMF 16x40 (107k units) on 1, 2,
+// 4, 8 and 16 blocks 9.8, 7.7, 5.5, 5.0 and 4.7 ms, 24x40 (245k) 24.0, 15.8,
+// 12.7, 12.9 ms on 2 to 16, 32x64 (702k) 57, 38 and 32 ms on 4 to 16.  One
+// block does the most work an SM; a large cluster ends soonest.
+constexpr int kHybClasses = 5;
+constexpr int kHybBlocks[kHybClasses] = {16, 8, 4, 2, 1};
+constexpr double kHybNs[kHybClasses] = {45, 52, 75, 95, 100};
+// The share of that which the mean instance takes (layered networks have a
+// fifth of GENRMF's rounds).
+constexpr double kHybMean = 0.5;
+
+// The class of an instance when the batch is to end after about `t` ns: the
+// fewest blocks that hold its vertices and end in time, or the most there are.
+int hybrid_class(int64_t n, int64_t units, double t, int least) {
+  for (int k = kHybClasses - 1; k >= least; --k)
+    if (n <= (int64_t)kHybBlocks[k] * kHybBlockVertices && (k == least || kHybNs[k] * (double)units <= t)) return k;
+  return -1;
+}
+
+// Capture the batch launch as a CUDA graph of concurrent launches, each
+// claiming its instances, largest first, from a list of its own:
+//   mixed (no knob of this file's kernel is set): the instances that fit one
+//     block's shared memory on the resident solver, the other sparse ones on
+//     the hybrid solver, each on the fewest blocks that end before the batch
+//     as a whole can;
+//   of the instances that are left, those of at least `cluster_units` units an
+//     8-block cluster each of this file's kernel, the others a block each.
+// Measured on GB300 on uneven instances (half GENRMF, a and b log-uniform in
+// [4, 32] x [4, 64], half layered networks), this file's kernel alone and now:
+//   21 instances 68 -> 8.3 ms, 100 122 -> 13 ms, 512 295 -> 38 ms, 2,048
+//   331 -> 88 ms, 4,096 361 -> 160 ms (p99 of an instance 155 -> 40 ms).
+// With every instance from 2^16 or 2^17 units on 16 blocks 512 take 92 and 70
+// ms, with none 68 ms.
 wbpr_status capture(wbpr_batch* b, int tile, int block, double alpha, int grr, long long max_rounds,
-                    double max_ms, int64_t cluster_units) {
+                    double max_ms, int64_t cluster_units, bool mixed) {
   if (b->exec && b->cap_tile == tile && b->cap_block == block && b->cap_alpha == alpha && b->cap_grr == grr &&
-      b->cap_cluster == cluster_units)
+      b->cap_cluster == cluster_units && b->cap_mixed == mixed && b->cap_rounds == max_rounds && b->cap_ms == max_ms)
     return WBPR_OK;
   if (b->exec) {
     cudaGraphExecDestroy(b->exec);
     b->exec = nullptr;
   }
-  int nbig = 0;
-  if (cluster_units >= 0)
-    while (nbig < b->count && b->size_sorted[(size_t)nbig] >= cluster_units) ++nbig;
+  // the lists, one after the other in `order`
+  enum { kHybrid, kResident = kHybrid + kHybClasses, kCluster, kBlock, kLists };
+  static_assert(kLists == wbpr_batch::kLaunches, "one claim counter a launch");
+  std::vector<int32_t> list[kLists];
+  const int64_t big_units = cluster_units > 0 ? cluster_units : kBatchClusterUnits;
+  int hyb_most[kHybClasses] = {};  // clusters at once
+  int least = kHybClasses;    // the largest cluster there is
+  for (int k = kHybClasses - 1; k >= 0; --k) {
+    hyb_most[k] = mixed ? hybrid_clusters(kHybBlocks[k]) : 0;
+    if (hyb_most[k] == 0) break;
+    least = k;
+  }
+  std::vector<int32_t> hyb;
+  for (int32_t id : b->host_order) {
+    const wbpr_batch::Shape& x = b->shape[(size_t)id];
+    if (mixed && resident_one_block(x.n, x.arcs)) list[kResident].push_back(id);
+    else if (least < kHybClasses && hybrid_takes(x.n, x.arcs, x.longer) && hybrid_class(x.n, x.units(), 0, least) >= 0)
+      hyb.push_back(id);
+    else list[cluster_units >= 0 && x.units() >= big_units ? kCluster : kBlock].push_back(id);
+  }
+  // the shortest time in which the SMs can do the work that it asks for
+  auto class_of = [&](int32_t id, double t) {
+    const wbpr_batch::Shape& x = b->shape[(size_t)id];
+    if (cluster_units > 0) t = x.units() >= cluster_units ? 0 : 1e30;
+    return hybrid_class(x.n, x.units(), t, least);
+  };
+  double t = 1e5;
+  for (; t < 1e12; t *= 1.1) {
+    double ns = 0;  // SM x time
+    for (int32_t id : hyb) {
+      const int k = class_of(id, t);
+      ns += kHybMean * kHybNs[k] * kHybBlocks[k] * (double)b->shape[(size_t)id].units();
+    }
+    for (int32_t id : list[kResident]) ns += kHybMean * kHybNs[kHybClasses - 1] * (double)b->shape[(size_t)id].units();
+    if (ns <= t * b->sms) break;
+  }
+  for (int32_t id : hyb) list[kHybrid + class_of(id, t)].push_back(id);
+  std::vector<int32_t> order;
+  int first[kLists], count[kLists];
+  for (int k = 0; k < kLists; ++k) {
+    first[k] = (int)order.size();
+    count[k] = (int)list[k].size();
+    order.insert(order.end(), list[k].begin(), list[k].end());
+  }
+  BCK(cudaMemcpyAsync(b->order, order.data(), 4 * order.size(), cudaMemcpyHostToDevice, b->stream));
+  BCK(cudaStreamSynchronize(b->stream));
+  // arc records of the clusters that run at once
+  int64_t rec_first[kHybClasses], rec_stride[kHybClasses], rec_total = 0;
+  int hyb_clusters[kHybClasses];
+  for (int k = 0; k < kHybClasses; ++k) {
+    rec_first[k] = rec_total;
+    rec_stride[k] = 0;
+    for (int32_t id : list[kHybrid + k]) rec_stride[k] = std::max(rec_stride[k], b->shape[(size_t)id].arcs);
+    hyb_clusters[k] = std::min(count[kHybrid + k], hyb_most[k]);
+    rec_total += hyb_clusters[k] * rec_stride[k];
+  }
+  if (b->rec_count < rec_total) {
+    // (an earlier, smaller block stays with the batch until it is destroyed)
+    wbpr_status st = balloc(b, &b->rec, (size_t)rec_total);
+    if (st) return st;
+    b->rec_count = rec_total;
+  }
   const void* fn = kernel_for(tile, false);
   int occ = 0;
   BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, 0));
@@ -431,11 +525,11 @@ wbpr_status capture(wbpr_batch* b, int tile, int block, double alpha, int grr, l
     wbpr::set_last_error("batch kernel does not fit on an SM");
     return WBPR_ERR_CUDA;
   }
-  const int grid = std::min<int64_t>((int64_t)b->sms * occ, std::max(1, b->count - nbig));
+  const int grid = (int)std::min<int64_t>((int64_t)b->sms * occ, std::max(1, count[kBlock]));
   cudaLaunchConfig_t big{};
   cudaLaunchAttribute big_attr[1];
   const void* fnb = kernel_for(tile, true);
-  if (nbig > 0) {
+  if (count[kCluster] > 0) {
     big.blockDim = dim3(block);
     big.stream = b->stream;
     big_attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -451,7 +545,7 @@ wbpr_status capture(wbpr_batch* b, int tile, int block, double alpha, int grr, l
       wbpr::set_last_error("batch cluster kernel does not fit");
       return WBPR_ERR_CUDA;
     }
-    big.gridDim = dim3(kBatchCluster * std::min(nbig, clusters));
+    big.gridDim = dim3(kBatchCluster * std::min(count[kCluster], clusters));
   }
   BatchParams bp;
   std::memset(&bp, 0, sizeof(bp));
@@ -459,8 +553,8 @@ wbpr_status capture(wbpr_batch* b, int tile, int block, double alpha, int grr, l
   bp.arc = b->arc;
   bp.arx = b->arx;
   bp.inst = b->inst;
-  bp.order = b->order;
-  bp.count = b->count;
+  bp.order = b->order + first[kBlock];
+  bp.count = count[kBlock];
   bp.h = b->h;
   bp.e = b->e;
   bp.rl_min = b->rl_min;
@@ -474,40 +568,81 @@ wbpr_status capture(wbpr_batch* b, int tile, int block, double alpha, int grr, l
   bp.flows = b->flows;
   bp.inst_ns = b->inst_ns;
   bp.inst_rounds = b->inst_rounds;
-  bp.next = b->next;
+  bp.next = b->next + kBlock;
   bp.gr_alpha = alpha;
   bp.gr_rounds = grr;
   bp.max_rounds = (int)std::min<long long>(max_rounds, 1 << 30);
   bp.budget_ns = (unsigned long long)(max_ms * 1e6);
-  BatchParams bpb = bp;  // the cluster branch: the first nbig instances of the order
-  bpb.count = nbig;
-  bpb.next = b->next_big;
-  bp.order = b->order + nbig;
-  bp.count = b->count - nbig;
+  BatchParams bpb = bp;
+  bpb.order = b->order + first[kCluster];
+  bpb.count = count[kCluster];
+  bpb.next = b->next + kCluster;
+  ResBatch rb{};
+  rb.row = b->row;
+  rb.arc = b->arc;
+  rb.arx = b->arx;
+  rb.inst = b->inst;
+  rb.order = b->order + first[kResident];
+  rb.count = count[kResident];
+  rb.next = b->next + kResident;
+  rb.lab = b->h;
+  rb.e = b->e;
+  rb.flows = b->flows;
+  rb.inst_ns = b->inst_ns;
+  rb.inst_rounds = b->inst_rounds;
+  rb.run.max_rounds = max_rounds;
+  rb.run.budget_ns = bp.budget_ns;
   cudaGraph_t graph = nullptr;
   BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-  cudaMemsetAsync(b->next, 0, 2 * sizeof(int), b->stream);  // next and next_big
-  if (nbig > 0) {
-    cudaEventRecord(b->fork, b->stream);
-    cudaStreamWaitEvent(b->side, b->fork, 0);
-    big.stream = b->side;
-    void* bargs[] = {&bpb};
-    cudaLaunchKernelExC(&big, fnb, bargs);
-    cudaEventRecord(b->join, b->side);
+  cudaError_t e = cudaMemsetAsync(b->next, 0, kLists * sizeof(int), b->stream);
+  cudaEventRecord(b->fork, b->stream);
+  auto branch = [&](int k, auto launch) {
+    cudaStreamWaitEvent(b->side[k], b->fork, 0);
+    const cudaError_t x = launch(b->side[k]);
+    if (e == cudaSuccess) e = x;
+    cudaEventRecord(b->join[k], b->side[k]);
+    cudaStreamWaitEvent(b->stream, b->join[k], 0);
+  };
+  for (int k = 0; k < kHybClasses; ++k) {
+    if (!hyb_clusters[k]) continue;
+    ResBatch hb = rb;
+    hb.order = b->order + first[kHybrid + k];
+    hb.count = count[kHybrid + k];
+    hb.next = b->next + kHybrid + k;
+    hb.rec = b->rec + rec_first[k];
+    hb.rec_stride = rec_stride[k];
+    branch(kHybrid + k, [&](cudaStream_t st) { return launch_hybrid_batch(hb, kHybBlocks[k], hyb_clusters[k], st); });
   }
-  void* args[] = {&bp};
-  if (bp.count > 0) cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, b->stream);
-  if (nbig > 0) cudaStreamWaitEvent(b->stream, b->join, 0);
-  BCK(cudaStreamEndCapture(b->stream, &graph));
-  cudaError_t e = cudaGraphInstantiate(&b->exec, graph, 0);
-  cudaGraphDestroy(graph);
-  BCK(e);
+  if (count[kResident] > 0)
+    branch(kResident, [&](cudaStream_t st) { return launch_resident_batch(rb, std::min(count[kResident], b->sms), st); });
+  if (count[kCluster] > 0)
+    branch(kCluster, [&](cudaStream_t st) {
+      big.stream = st;
+      void* args[] = {&bpb};
+      return cudaLaunchKernelExC(&big, fnb, args);
+    });
+  if (count[kBlock] > 0) {
+    void* args[] = {&bp};
+    const cudaError_t x = cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, b->stream);
+    if (e == cudaSuccess) e = x;
+  }
+  const cudaError_t end = cudaStreamEndCapture(b->stream, &graph);
+  if (e == cudaSuccess) e = end;
+  if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec, graph, 0);
+  if (graph) cudaGraphDestroy(graph);
+  if (e != cudaSuccess) {
+    b->exec = nullptr;
+    wbpr::set_last_error(std::string("batch capture: ") + cudaGetErrorString(e));
+    return WBPR_ERR_CUDA;
+  }
   b->cap_tile = tile;
   b->cap_block = block;
   b->cap_alpha = alpha;
   b->cap_grr = grr;
   b->cap_cluster = cluster_units;
-  b->cap_nbig = nbig;
+  b->cap_mixed = mixed;
+  b->cap_rounds = max_rounds;
+  b->cap_ms = max_ms;
   return WBPR_OK;
 }
 
@@ -566,14 +701,21 @@ wbpr_status wbpr_batch_create(const wbpr_csr* graphs, int32_t count, wbpr_batch*
   TRYBC(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
   TRYBC(cudaEventCreate(&b->ev0));
   TRYBC(cudaEventCreate(&b->ev1));
-  TRYBC(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking));
   TRYBC(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
-  TRYBC(cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming));
+  {
+    int low = 0, high = 0;
+    TRYBC(cudaDeviceGetStreamPriorityRange(&low, &high));
+    for (int k = 0; k < wbpr_batch::kSides; ++k) {
+      // the larger clusters first: they need as many free SMs at once
+      TRYBC(cudaStreamCreateWithPriority(&b->side[k], cudaStreamNonBlocking, std::min(low, high + k)));
+      TRYBC(cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming));
+    }
+  }
   // concatenate the instances' BCSR16 rows with global ids
   std::vector<int32_t> row((size_t)tn + 1);
   std::vector<int32_t> arc(2 * (size_t)tm), arx(2 * (size_t)tm);
   std::vector<BatchInst> inst((size_t)count);
-  std::vector<int64_t> size((size_t)count);
+  b->shape.resize((size_t)count);
   int64_t vb = 0, ab = 0;
   for (int i = 0; i < count; ++i) {
     wbpr::Bcsr16 r;
@@ -588,16 +730,17 @@ wbpr_status wbpr_batch_create(const wbpr_csr* graphs, int32_t count, wbpr_batch*
       arx[2 * (ab + a) + 1] = r.arx[2 * a + 1];
     }
     inst[i] = BatchInst{(int)vb, n, (int)(vb + graphs[i].source), (int)(vb + graphs[i].sink)};
-    size[i] = n + na;
+    int64_t longer = 0;
+    for (int u = 0; u < n; ++u) longer += r.row[u + 1] - r.row[u] > kLightDeg;
+    b->shape[(size_t)i] = {n, na, longer};
     vb += n;
     ab += na;
   }
   row[(size_t)tn] = (int32_t)ab;
-  std::vector<int32_t> order((size_t)count);
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return size[a] > size[c]; });
-  b->size_sorted.resize((size_t)count);
-  for (int i = 0; i < count; ++i) b->size_sorted[(size_t)i] = size[(size_t)order[(size_t)i]];
+  b->host_order.resize((size_t)count);
+  std::iota(b->host_order.begin(), b->host_order.end(), 0);
+  std::stable_sort(b->host_order.begin(), b->host_order.end(),
+                   [&](int a, int c) { return b->shape[(size_t)a].units() > b->shape[(size_t)c].units(); });
   TRYB(balloc(b, &b->row, (size_t)tn + 1));
   TRYB(balloc(b, &b->arc, (size_t)tm));
   TRYB(balloc(b, &b->arx, (size_t)tm));
@@ -609,15 +752,13 @@ wbpr_status wbpr_batch_create(const wbpr_csr* graphs, int32_t count, wbpr_batch*
     TRYBC(cudaMemcpy(b->arx, arx.data(), 4 * arx.size(), cudaMemcpyHostToDevice));
   }
   TRYBC(cudaMemcpy(b->inst, inst.data(), sizeof(BatchInst) * inst.size(), cudaMemcpyHostToDevice));
-  TRYBC(cudaMemcpy(b->order, order.data(), 4 * order.size(), cudaMemcpyHostToDevice));
   int** vec[] = {&b->h, &b->e, &b->rl_min, &b->rl_left, &b->esnap, &b->lq[0], &b->lq[1], &b->qraw,
                  &b->fr[0], &b->fr[1]};
   for (int** p : vec) TRYB(balloc(b, p, (size_t)tn));
   TRYB(balloc(b, &b->flows, (size_t)count));
   TRYB(balloc(b, &b->inst_ns, (size_t)count));
   TRYB(balloc(b, &b->inst_rounds, (size_t)count));
-  TRYB(balloc(b, &b->next, 2));
-  b->next_big = b->next + 1;
+  TRYB(balloc(b, &b->next, wbpr_batch::kLaunches));
   b->host_flows.resize((size_t)count);
 #undef TRYB
 #undef TRYBC
@@ -651,8 +792,9 @@ wbpr_status wbpr_batch_solve(wbpr_batch* b, const wbpr_tuning* tu, int64_t* flow
   const double max_ms = tu->max_ms > 0 ? tu->max_ms : 120000.0;
   BCK(cudaSetDevice(b->device));
   if (tu->batch_cluster < -1) return WBPR_ERR_INVALID_ARG;
-  const int64_t cl = tu->batch_cluster == 0 ? kBatchClusterUnits : tu->batch_cluster;
-  wbpr_status st = capture(b, tile, block, alpha, grr, tu->max_rounds, max_ms, cl);
+  // the defaults: the resident and hybrid solvers have none of these knobs
+  const bool mixed = tile == 8 && block == 512 && alpha == 1.0 && !tu->gr_rounds && tu->batch_cluster >= 0;
+  wbpr_status st = capture(b, tile, block, alpha, grr, tu->max_rounds, max_ms, tu->batch_cluster, mixed);
   if (st) return st;
   BCK(cudaEventRecord(b->ev0, b->stream));
   BCK(cudaGraphLaunch(b->exec, b->stream));

@@ -1681,23 +1681,15 @@ wbpr_status run_resident(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* laun
       if (st) return st;
     }
     if (launch_ms) CK(cudaEventRecord(g->ev2, g->stream));
-    cudaError_t e;
-    if (g->res_cluster) {
-      ResParams p{};
-      p.in = in;
-      p.out = g->res_out;
-      p.max_rounds = rc.max_rounds;
-      p.budget_ns = rc.budget_ns;
-      e = launch_resident(p, g->avg_deg < 20 ? 8 : 32, g->res_cluster, g->stream);
-    } else {
-      HybParams p{};
-      p.in = in;
-      p.out = g->res_out;
-      p.rec = g->hyb_rec;
-      p.max_rounds = rc.max_rounds;
-      p.budget_ns = rc.budget_ns;
-      e = launch_hybrid(p, g->stream);
-    }
+    ResParams p{};
+    p.in = in;
+    p.to.out = g->res_out;
+    p.run.max_rounds = rc.max_rounds;
+    p.run.budget_ns = rc.budget_ns;
+    p.keep = true;
+    p.rec = g->hyb_rec;
+    const cudaError_t e = g->res_cluster ? launch_resident(p, g->avg_deg < 20 ? 8 : 32, g->res_cluster, g->stream)
+                                         : launch_hybrid(p, g->stream);
     if (e != cudaSuccess) {
       cudaGetLastError();  // no such cluster on this device: the persistent kernel takes the graph
       g->res_cluster = 0;

@@ -53,7 +53,7 @@ struct HPart {
   unsigned a0;                      // shared-memory address of the block's memory
   unsigned a_list, a_lab, a_e, a_ex, a_row;  // offsets from it
   int4* rec;
-  int rank, cs;
+  int rank, cs, shift;     // cs = 1 << shift blocks
   int groups;
   int n;
   int row0;                // arc number of record 0
@@ -67,9 +67,9 @@ struct HPart {
   // the vertex in a slot of this block (>= n: the slot is empty)
   __device__ __forceinline__ int vertex(int s) const {
     const int l = s >> 2 & 31, q = (s & 3) * 32 + (l & 7) * 4 + (l >> 3);
-    return (q * groups + (s >> 7)) * kResMaxCluster + rank;
+    return (q * groups + (s >> 7)) * cs + rank;
   }
-  __device__ __forceinline__ int code(int v) const { return v % kResMaxCluster << 16 | slot(v / kResMaxCluster); }
+  __device__ __forceinline__ int code(int v) const { return (v & (cs - 1)) << 16 | slot(v >> shift); }
 };
 
 __device__ __forceinline__ int4 lds128(unsigned a) {
@@ -105,6 +105,7 @@ __device__ void setup(const ResInstance& in, int4* rec, char* sm, HPart& P) {
   P.c = c;
   P.cs = (int)cl_size();
   P.rank = (int)cl_rank();
+  P.shift = 31 - __clz(P.cs);
   P.n = in.n;
   P.rec = rec;
   P.row0 = row_at(in, 0);
@@ -267,7 +268,7 @@ __device__ __forceinline__ void bfs_expand(const ResInstance& in, const HPart& P
 // Exact distances to (DIR 0) or from (DIR 1) t, as in the resident solver.
 // The root's row, which may be the graph's longest, is shared by all blocks.
 template <int DIR>
-__device__ int bfs_hybrid(const HybParams& p, const HPart& P, int& seq, Count& ct) {
+__device__ int bfs_hybrid(const ResParams& p, const HPart& P, int& seq, Count& ct) {
   const ResInstance& in = p.in;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int i = threadIdx.x; i < 128 * P.groups; i += blockDim.x) {
@@ -285,7 +286,7 @@ __device__ int bfs_hybrid(const HybParams& p, const HPart& P, int& seq, Count& c
   List list(P);
   for (;;) {
     bool did = false;
-    for (int k = 0; k < p.bsub; ++k) {
+    for (int k = 0; k < p.run.bsub; ++k) {
       bool now = false;
       const auto expand = [&](int u) { bfs_expand<kTile, DIR>(in, P, u, ct); };
       for (int g = wid; g < P.groups; g += nw) {
@@ -301,10 +302,10 @@ __device__ int bfs_hybrid(const HybParams& p, const HPart& P, int& seq, Count& c
       }
       list.drain<kTile>(expand);
       did |= now;
-      if (k + 1 < p.bsub && !__syncthreads_or(now)) break;
+      if (k + 1 < p.run.bsub && !__syncthreads_or(now)) break;
     }
     if (!any_work<true>(P.c, P.a0, P.cs, did, seq)) return levels;
-    levels += p.bsub;
+    levels += p.run.bsub;
   }
 }
 
@@ -414,7 +415,7 @@ __device__ bool push_step(const ResInstance& in, const HPart& P, Count& ct) {
   return did;
 }
 
-__device__ void solve_hybrid(const HybParams& p, const HPart& P, ResOut* out) {
+__device__ void solve_hybrid(const ResParams& p, const HPart& P) {
   const ResInstance& in = p.in;
   Count ct;
   int seq = 0, grs = 0, rounds = 0, since = 0, err = 0, total_levels = 0;
@@ -452,10 +453,10 @@ __device__ void solve_hybrid(const HybParams& p, const HPart& P, ResOut* out) {
       const bool did = push_step(in, P, ct);
       if (P.rank == 0 && threadIdx.x < P.cs) {
         const unsigned to = Smem::at(P.a0, threadIdx.x);
-        const bool out_of_time = (unsigned long long)(clock64() - clk0) >= p.budget_ns >> 1 && time_past(t0, p.budget_ns);
-        if ((p.max_rounds > 0 && rounds >= p.max_rounds) || out_of_time)
+        const bool out_of_time = (unsigned long long)(clock64() - clk0) >= p.run.budget_ns >> 1 && time_past(t0, p.run.budget_ns);
+        if ((p.run.max_rounds > 0 && rounds >= p.run.max_rounds) || out_of_time)
           Smem::st(to + (unsigned)offsetof(ResCtl, stop), seq + 1);
-        if (since >= 8 && (clock64() - gr_end) * 16 >= gr_len * p.grp) Smem::st(to + (unsigned)offsetof(ResCtl, gr), seq + 1);
+        if (since >= 8 && (clock64() - gr_end) * 16 >= gr_len * p.run.grp) Smem::st(to + (unsigned)offsetof(ResCtl, gr), seq + 1);
       }
       if (!any_work<true>(P.c, P.a0, P.cs, did, seq)) break;
       if (*(volatile int*)&P.c->stop == seq) {
@@ -467,7 +468,7 @@ __device__ void solve_hybrid(const HybParams& p, const HPart& P, ResOut* out) {
       ++since;
     }
   }
-  write_back(in, P);
+  if (p.keep) write_back(in, P);
   if (in.mode != kModeBfsOnly) {
     int str = 0;
     for (int i = threadIdx.x; i < 128 * P.groups; i += blockDim.x)
@@ -479,45 +480,62 @@ __device__ void solve_hybrid(const HybParams& p, const HPart& P, ResOut* out) {
       for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(kFull, v[k], o);
       if (lane == 0 && v[k]) Smem::add64(Smem::at(P.a0, 0) + (unsigned)offsetof(ResCtl, sum) + 8 * k, v[k]);
     }
-    if (P.tl >= 0 && threadIdx.x == 0) out->flow = (int)lds32(P.a0 + P.a_e + 4 * P.tl);
     Smem::sync();
   }
-  if (P.rank == 0 && threadIdx.x == 0) {
-    Stats s{};
-    s.arcs_scanned = P.c->sum[0];
-    s.bfs_arcs = P.c->sum[1];
-    s.pushes = P.c->sum[2];
-    s.relabels = P.c->sum[3];
-    s.vertex_visits = P.c->sum[4];
-    s.stranded = (int)P.c->sum[5];
-    s.rounds = rounds;
-    s.grs = grs;
-    s.bfs_levels = total_levels;
-    const unsigned long long ns = gtime() - t0;
-    s.gr_ns = (unsigned long long)((double)ns * (double)gr_all / (double)(clock64() - clk0));
-    s.push_ns = s.round_ns = ns - s.gr_ns;
-    out->st = s;
-    out->err = err;
-  }
+  report(p.to, P.c, P.rank, in.mode != kModeBfsOnly && P.tl >= 0, P.tl >= 0 ? (int)lds32(P.a0 + P.a_e + 4 * P.tl) : 0, err, rounds, grs, total_levels, gtime() - t0,
+         (double)gr_all / (double)(clock64() - clk0));
 }
 
 extern __shared__ __align__(16) char hyb_smem[];
 
-__global__ void __launch_bounds__(kResThreads) pr_hybrid(const __grid_constant__ HybParams p) {
+__global__ void __launch_bounds__(kResThreads) pr_hybrid(const __grid_constant__ ResParams p) {
   HPart P;
   setup(p.in, p.rec, hyb_smem, P);
   build_records(p.in, P);
   Smem::sync();
-  solve_hybrid(p, P, p.out);
+  solve_hybrid(p, P);
+}
+
+__global__ void __launch_bounds__(kResThreads) pr_hybrid_batch(const __grid_constant__ ResBatch b) {
+  ResParams p;
+  int4* rec = b.rec + b.rec_stride * (blockIdx.x / cl_size());
+  while (claim<true>(b, hyb_smem, p, rec)) {
+    HPart P;
+    setup(p.in, p.rec, hyb_smem, P);
+    build_records(p.in, P);
+    Smem::sync();
+    solve_hybrid(p, P);
+  }
 }
 
 }  // namespace
 
-cudaError_t launch_hybrid(const HybParams& p0, cudaStream_t st) {
-  HybParams p = p0;
-  p.bsub = kHybBfsLevels;
-  p.grp = kHybGrShare;
+cudaError_t launch_hybrid(const ResParams& p0, cudaStream_t st) {
+  ResParams p = p0;
+  p.run.bsub = kHybBfsLevels;
+  p.run.grp = kHybGrShare;
   return launch_cluster<pr_hybrid>(p, kResMaxCluster, st);
+}
+
+int hybrid_clusters(int blocks) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[1];
+  if (cluster_config<pr_hybrid_batch>(blocks, 1024, nullptr, &cfg, at) != cudaSuccess) return 0;
+  int n = 0, dev = 0, sms = 0;
+  if (blocks == 1) {
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    return sms;
+  }
+  if (cudaOccupancyMaxActiveClusters(&n, (const void*)pr_hybrid_batch, &cfg) != cudaSuccess) n = 0;
+  cudaGetLastError();
+  return n;
+}
+
+cudaError_t launch_hybrid_batch(const ResBatch& b0, int blocks, int clusters, cudaStream_t st) {
+  ResBatch b = b0;
+  b.run.bsub = kHybBfsLevels;
+  b.run.grp = kHybGrShare;
+  return launch_cluster<pr_hybrid_batch>(b, blocks, st, clusters);
 }
 
 }  // namespace wbpr_dev

@@ -106,7 +106,7 @@ __device__ __forceinline__ int owner_of(const ResCtl* c, int cs, int v) {
 // Splits the instance over the cluster and lays out the memory; false when a
 // block's share does not fit (all blocks agree).
 template <bool CL>
-__device__ bool setup(const ResInstance& in, int smem_bytes, char* sm, Part& P) {
+__device__ bool setup(const ResInstance& in, char* sm, Part& P) {
   ResCtl* c = (ResCtl*)sm;
   P.c = c;
   P.cs = CL ? (int)cl_size() : 1;
@@ -142,7 +142,7 @@ __device__ bool setup(const ResInstance& in, int smem_bytes, char* sm, Part& P) 
   q += 4 * (size_t)slots;
   P.ex = (unsigned short*)q;
   q += 2 * (size_t)slots;
-  if (q > sm + smem_bytes || slots > kResMaxVertices || namax > kResMaxArcs) return false;
+  if (q > sm + kResSmem || slots > kResMaxVertices || namax > kResMaxArcs) return false;
   P.a0 = sm_addr(sm);
   P.a_rec = sm_addr(P.rec) - P.a0;
   P.a_ve = sm_addr(P.ve) - P.a0;
@@ -278,7 +278,7 @@ __device__ int bfs_resident(const ResParams& p, Part& P, int& seq, Count& ct) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (;;) {
     bool did = false;
-    for (int k = 0; k < p.bsub; ++k) {
+    for (int k = 0; k < p.run.bsub; ++k) {
       bool now = false;
       for (int g = wid; g < P.groups; g += nw) {
         const int i = g * 32 + lane;
@@ -309,10 +309,10 @@ __device__ int bfs_resident(const ResParams& p, Part& P, int& seq, Count& ct) {
         }
       }
       did |= now;
-      if (k + 1 < p.bsub && !__syncthreads_or(now)) break;
+      if (k + 1 < p.run.bsub && !__syncthreads_or(now)) break;
     }
     if (!any_work<CL>(P.c, P.a0, P.cs, did, seq)) return levels;
-    levels += p.bsub;
+    levels += p.run.bsub;
   }
 }
 
@@ -434,7 +434,7 @@ __device__ __forceinline__ bool push_step(const Part& P, Count& ct) {
 }
 
 template <int W, bool CL>
-__device__ void solve_resident(const ResParams& p, Part& P, ResOut* out) {
+__device__ void solve_resident(const ResParams& p, Part& P) {
   const ResInstance& in = p.in;
   Count ct;
   int seq = 0, grs = 0, rounds = 0, since = 0, err = 0, total_levels = 0;
@@ -478,10 +478,10 @@ __device__ void solve_resident(const ResParams& p, Part& P, ResOut* out) {
       if (P.rank == 0 && threadIdx.x < P.cs) {
         const unsigned to = Sh<CL>::at(P.a0, threadIdx.x);
         // the cycle counter first (cheaper to read; an SM does over half a cycle per ns)
-        const bool out_of_time = (unsigned long long)(clock64() - clk0) >= p.budget_ns >> 1 && time_past(t0, p.budget_ns);
-        if ((p.max_rounds > 0 && rounds >= p.max_rounds) || out_of_time)
+        const bool out_of_time = (unsigned long long)(clock64() - clk0) >= p.run.budget_ns >> 1 && time_past(t0, p.run.budget_ns);
+        if ((p.run.max_rounds > 0 && rounds >= p.run.max_rounds) || out_of_time)
           Sh<CL>::st(to + (unsigned)offsetof(ResCtl, stop), seq + 1);
-        if (since >= 8 && (clock64() - gr_end) * 16 >= gr_len * p.grp) Sh<CL>::st(to + (unsigned)offsetof(ResCtl, gr), seq + 1);
+        if (since >= 8 && (clock64() - gr_end) * 16 >= gr_len * p.run.grp) Sh<CL>::st(to + (unsigned)offsetof(ResCtl, gr), seq + 1);
       }
       // the labels are valid after every step, so no active vertex means a
       // maximum preflow
@@ -495,7 +495,7 @@ __device__ void solve_resident(const ResParams& p, Part& P, ResOut* out) {
       ++since;
     }
   }
-  write_back(in, P);
+  if (p.keep) write_back(in, P);
   // counters: warps into the block's words, blocks into the first block's
   if (in.mode != kModeBfsOnly) {
     int str = 0;
@@ -508,26 +508,10 @@ __device__ void solve_resident(const ResParams& p, Part& P, ResOut* out) {
       for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(kFull, v[k], o);
       if (lane == 0 && v[k]) Sh<CL>::add64(Sh<CL>::at(P.a0, 0) + (unsigned)offsetof(ResCtl, sum) + 8 * k, v[k]);
     }
-    if (P.tl >= 0 && threadIdx.x == 0) out->flow = P.ve[P.tl].y;
     Sh<CL>::sync();
   }
-  if (P.rank == 0 && threadIdx.x == 0) {
-    Stats s{};
-    s.arcs_scanned = P.c->sum[0];
-    s.bfs_arcs = P.c->sum[1];
-    s.pushes = P.c->sum[2];
-    s.relabels = P.c->sum[3];
-    s.vertex_visits = P.c->sum[4];
-    s.stranded = (int)P.c->sum[5];
-    s.rounds = rounds;
-    s.grs = grs;
-    s.bfs_levels = total_levels;
-    const unsigned long long ns = gtime() - t0;
-    s.gr_ns = (unsigned long long)((double)ns * (double)gr_all / (double)(clock64() - clk0));
-    s.push_ns = s.round_ns = ns - s.gr_ns;
-    out->st = s;
-    out->err = err;
-  }
+  report(p.to, P.c, P.rank, in.mode != kModeBfsOnly && P.tl >= 0, P.tl >= 0 ? P.ve[P.tl].y : 0, err, rounds, grs, total_levels, gtime() - t0,
+         (double)gr_all / (double)(clock64() - clk0));
 }
 
 extern __shared__ __align__(16) char res_smem[];
@@ -535,12 +519,25 @@ extern __shared__ __align__(16) char res_smem[];
 template <int W, bool CL>
 __global__ void __launch_bounds__(kResThreads) pr_resident(const __grid_constant__ ResParams p) {
   Part P;
-  if (!setup<CL>(p.in, p.smem_bytes, res_smem, P)) {
-    if (P.rank == 0 && threadIdx.x == 0) p.out->err = kResNoFit;
+  if (!setup<CL>(p.in, res_smem, P)) {
+    if (P.rank == 0 && threadIdx.x == 0) p.to.out->err = kResNoFit;
     return;
   }
   load<W, CL>(p.in, P);
-  solve_resident<W, CL>(p, P, p.out);
+  solve_resident<W, CL>(p, P);
+}
+
+__global__ void __launch_bounds__(kResThreads) pr_resident_batch(const __grid_constant__ ResBatch b) {
+  ResParams p;
+  while (claim<false>(b, res_smem, p, nullptr)) {
+    Part P;
+    if (!setup<false>(p.in, res_smem, P)) {  // the host puts no such instance here
+      if (threadIdx.x == 0) *p.to.flow = -1;
+      continue;
+    }
+    load<8, false>(p.in, P);
+    solve_resident<8, false>(p, P);
+  }
 }
 
 }  // namespace
@@ -556,12 +553,23 @@ int resident_cluster(long long n, long long na) {
 
 cudaError_t launch_resident(const ResParams& p0, int tile, int cluster, cudaStream_t st) {
   ResParams p = p0;
-  p.smem_bytes = kResSmem;
-  // measured on GB300: see the head of this file
-  p.bsub = cluster == 1 ? 1 : kResBfsLevels;
-  p.grp = kResGrShare;
+    p.run.bsub = cluster == 1 ? 1 : kResBfsLevels;
+  p.run.grp = kResGrShare;
   if (cluster == 1) return tile < 32 ? launch_cluster<pr_resident<8, false>>(p, 1, st) : launch_cluster<pr_resident<32, false>>(p, 1, st);
   return tile < 32 ? launch_cluster<pr_resident<8, true>>(p, cluster, st) : launch_cluster<pr_resident<32, true>>(p, cluster, st);
+}
+
+bool resident_one_block(long long n, long long na) {
+  const long long slots = 32 * (n > kResThreads ? (n + 31) / 32 : kResThreads / 32);
+  return (long long)((sizeof(ResCtl) + 15) & ~15u) + kResArcBytes * na + kResVertexBytes * slots <= kResSmem && slots <= kResMaxVertices &&
+         na <= kResMaxArcs;
+}
+
+cudaError_t launch_resident_batch(const ResBatch& b0, int blocks, cudaStream_t st) {
+  ResBatch b = b0;
+  b.run.bsub = 1;
+  b.run.grp = kResGrShare;
+  return launch_cluster<pr_resident_batch>(b, 1, st, blocks);
 }
 
 }  // namespace wbpr_dev

@@ -21,6 +21,7 @@ struct ResCtl {
   int busy[2];                    // number of the last barrier before which some block had work, by parity
   int stop;                       // number of the barrier after which every block stops: budget exhausted
   int gr;                         // number of the barrier after which every block relabels globally
+  int item;                       // the claimed instance of a batch
   unsigned long long sum[8];      // counters
 };
 
@@ -122,10 +123,75 @@ __device__ __forceinline__ int row_at(const ResInstance& in, int v) {
   return in.row ? __ldg(in.row + in.vbase + v) : __ldg(in.frow + v) + __ldg(in.rrow + v);
 }
 
-// Launches one cluster of `blocks` blocks (1: no cluster) with the whole shared
-// memory of an SM each.
-template <auto Fn, class Prm>
-cudaError_t launch_cluster(const Prm& p, int blocks, cudaStream_t st, int clusters = 1) {
+// Writes the results of one solve (called by every thread of the cluster
+// behind the barrier after which c->sum is complete); `mine`: this block owns
+// t, whose excess is `flow`.
+__device__ __forceinline__ void report(const ResReport& to, const ResCtl* c, int rank, bool mine, int flow, int err, int rounds, int grs,
+                                       int levels, unsigned long long ns, double gr_share) {
+  if (threadIdx.x != 0) return;
+  if (mine) {
+    if (to.out) to.out->flow = flow;
+    else *to.flow = err ? -1 : flow;
+  }
+  if (rank != 0) return;
+  if (!to.out) {
+    *to.ns = ns;
+    *to.rounds = rounds;
+    return;
+  }
+  Stats s{};
+  s.arcs_scanned = c->sum[0];
+  s.bfs_arcs = c->sum[1];
+  s.pushes = c->sum[2];
+  s.relabels = c->sum[3];
+  s.vertex_visits = c->sum[4];
+  s.stranded = (int)c->sum[5];
+  s.rounds = rounds;
+  s.grs = grs;
+  s.bfs_levels = levels;
+  s.gr_ns = (unsigned long long)((double)ns * gr_share);
+  s.push_ns = s.round_ns = ns - s.gr_ns;
+  to.out->st = s;
+  to.out->err = err;
+}
+
+// The next instance of a batch for this block or cluster; false when none is
+// left.  A barrier: the memory of the last instance is free afterwards.
+template <bool CL>
+__device__ bool claim(const ResBatch& b, char* sm, ResParams& p, int4* rec) {
+  ResCtl* c = (ResCtl*)sm;
+  const unsigned rank = CL ? cl_rank() : 0, cs = CL ? cl_size() : 1;
+  Sh<CL>::sync();  // every block is done with the last instance (and has started)
+  if (rank == 0 && threadIdx.x == 0) {
+    const int i = atomicAdd(b.next, 1);
+    for (unsigned k = 0; k < cs; ++k) Sh<CL>::st(Sh<CL>::at(sm_addr(sm), k) + (unsigned)offsetof(ResCtl, item), i);
+  }
+  Sh<CL>::sync();
+  const int i = *(volatile int*)&c->item;
+  if (i >= b.count) return false;
+  const int id = __ldg(b.order + i);
+  const ResInst in = b.inst[id];
+  p.in = ResInstance{};
+  p.in.n = in.n;
+  p.in.vbase = in.vbase;
+  p.in.s = in.s - in.vbase;
+  p.in.t = in.t - in.vbase;
+  p.in.mode = kModeFresh;
+  p.in.row = b.row;
+  p.in.arc = b.arc;
+  p.in.arx = b.arx;
+  p.in.lab = b.lab;
+  p.in.e = b.e;
+  p.to = ResReport{nullptr, b.flows + id, b.inst_ns + id, b.inst_rounds + id};
+  p.run = b.run;
+  p.keep = false;
+  p.rec = rec;
+  return true;
+}
+
+// The launch configuration of `clusters` clusters of `blocks` blocks each, with the whole shared memory of an SM for every block.
+template <auto Fn>
+cudaError_t cluster_config(int blocks, int clusters, cudaStream_t st, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
   static std::mutex mu;
   static bool ready[64] = {false};  // of this kernel, by device
   int dev = 0;
@@ -135,21 +201,27 @@ cudaError_t launch_cluster(const Prm& p, int blocks, cudaStream_t st, int cluste
     std::lock_guard<std::mutex> lk(mu);
     if (dev >= 64 || !ready[dev]) {
       if ((e = cudaFuncSetAttribute((const void*)Fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem)) != cudaSuccess) return e;
-      if (blocks > 1 && (e = cudaFuncSetAttribute((const void*)Fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
+      if ((e = cudaFuncSetAttribute((const void*)Fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
       if (dev < 64) ready[dev] = true;
     }
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(blocks * clusters);
-  cfg.blockDim = dim3(kResThreads);
-  cfg.dynamicSmemBytes = kResSmem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cfg->gridDim = dim3(blocks * clusters);
+  cfg->blockDim = dim3(kResThreads);
+  cfg->dynamicSmemBytes = kResSmem;
+  cfg->stream = st;
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = blocks;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = blocks > 1 ? 1 : 0;
+  cfg->attrs = at;
+  cfg->numAttrs = blocks > 1 ? 1 : 0;  // a block without one is a cluster of its own
+  return cudaSuccess;
+}
+template <auto Fn, class Prm>
+cudaError_t launch_cluster(const Prm& p, int blocks, cudaStream_t st, int clusters = 1) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[1];
+  const cudaError_t e = cluster_config<Fn>(blocks, clusters, st, &cfg, at);
+  if (e != cudaSuccess) return e;
   void* args[] = {(void*)&p};
   return cudaLaunchKernelExC(&cfg, (const void*)Fn, args);
 }

@@ -47,14 +47,50 @@ struct ResInstance {
   int* e;      // excess out (state mode: in and out)
 };
 
-struct ResParams {
-  ResInstance in;
-  ResOut* out;
+// Where the results go.
+struct ResReport {
+  ResOut* out;  // nullptr: the three words below instead (an instance of a batch)
+  long long* flow;
+  unsigned long long* ns;
+  int* rounds;
+};
+
+struct ResRun {
   long long max_rounds;
   unsigned long long budget_ns;
-  int smem_bytes;
   int bsub;   // BFS levels between two cluster barriers
   int grp;    // global relabel when the rounds since the last one took grp / 16 x its time
+};
+
+struct ResParams {
+  ResInstance in;
+  ResReport to;
+  ResRun run;
+  bool keep;     // write residuals, labels and excess back
+  int4* rec;     // hybrid only: one record a residual arc (hybrid.cu)
+};
+
+// Instances of a batch, claimed one after the other by the blocks or clusters
+// of one launch.
+struct ResInst {
+  int vbase, n, s, t;  // s and t are global vertex ids
+};
+struct ResBatch {
+  const int* row;
+  int2* arc;
+  const int2* arx;
+  const ResInst* inst;
+  const int* order;  // this launch's instances, largest first
+  int count;
+  int* next;         // claim counter, zero at launch
+  int* lab;
+  int* e;
+  long long* flows;
+  unsigned long long* inst_ns;
+  int* inst_rounds;
+  ResRun run;
+  int4* rec;             // hybrid only: `rec_stride` records a cluster
+  long long rec_stride;
 };
 
 // The hybrid solver: the vertices in the shared memory of a 16-block cluster,
@@ -62,17 +98,8 @@ struct ResParams {
 constexpr int kHybVertexBytes = 12;     // label, excess, expanded label
 constexpr int kHybRowBytes = 8;         // the row, where there is room for it
 constexpr int kHybListBytes = 32 * 512;  // 256 slots a warp
-constexpr int kHybMaxVertices = kResMaxCluster * ((kResSmem - kResHeader - kHybListBytes) / kHybVertexBytes / 128 * 128);
-
-struct HybParams {
-  ResInstance in;
-  ResOut* out;
-  int4* rec;  // one record a residual arc: (hybrid.cu)
-  long long max_rounds;
-  unsigned long long budget_ns;
-  int bsub;
-  int grp;
-};
+constexpr int kHybBlockVertices = (kResSmem - kResHeader - kHybListBytes) / kHybVertexBytes / 128 * 128;
+constexpr int kHybMaxVertices = kResMaxCluster * kHybBlockVertices;
 
 // Whether the hybrid solver should take a graph: n vertices, na residual arcs,
 // `longer` of its rows longer than kLightDeg arcs.
@@ -83,7 +110,10 @@ struct HybParams {
 inline bool hybrid_takes(long long n, long long na, long long longer) {
   return n <= kHybMaxVertices && na < 20 * n && longer <= 2 + n / 256;
 }
-cudaError_t launch_hybrid(const HybParams& p, cudaStream_t st);
+cudaError_t launch_hybrid(const ResParams& p, cudaStream_t st);
+// Clusters of `blocks` (a power of two) of the hybrid solver that run at once.
+int hybrid_clusters(int blocks);
+cudaError_t launch_hybrid_batch(const ResBatch& b, int blocks, int clusters, cudaStream_t st);
 
 // Above this many vertices and residual arcs a graph that both could take goes
 // to the hybrid solver: its vertices are dealt to the blocks one by one, the
@@ -95,5 +125,8 @@ constexpr long long kResPreferUnits = 1 << 17;
 // power of two whose shared memory holds it, or 0.
 int resident_cluster(long long n, long long na);
 cudaError_t launch_resident(const ResParams& p, int tile, int cluster, cudaStream_t st);
+// Whether one block holds the graph (exact).
+bool resident_one_block(long long n, long long na);
+cudaError_t launch_resident_batch(const ResBatch& b, int blocks, cudaStream_t st);
 
 }  // namespace wbpr_dev
