@@ -94,3 +94,30 @@ def test_resident_budgets_and_new_terminals():
         cap = np.random.default_rng(1).integers(0, 500, g.m).astype(np.int32)
         d.set_capacities(cap)
         assert d.solve("vc", g.s, g.t).flow == oracle.dinic(g.n, g.off, g.dst, cap, g.s, g.t)
+
+
+@pytest.mark.parametrize("make", [lambda: W.gen_genrmf(6, 9, 1, 10000, 2), lambda: W.gen_rmat(13, 16, seed=8),
+                                  lambda: W.gen_grid(80, 90, 3), lambda: W.gen_rmat(14, 16, seed=9)])
+def test_caller_buffers_on_either_solver(make):
+    """wbpr_solve_bcsr_noalloc on graphs of one block, of a cluster and too
+    large for one, twice, and with the same buffers refused in between."""
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    g = make()
+    off, dst, cap, back = W.build_bcsr(g)
+    arc = torch.from_numpy(np.stack([dst, cap], 1)).cuda()
+    row = torch.from_numpy(off).cuda()
+    flow = C.c_int64(-1)
+
+    def solve(twins, algo):
+        arx = torch.from_numpy(np.stack([twins, cap], 1).astype(np.int32)).cuda()
+        return W.lib().wbpr_solve_bcsr_noalloc(g.n, 2 * g.m, row.data_ptr(), arc.data_ptr(), arx.data_ptr(), g.s, g.t, algo,
+                                               None, C.byref(flow))
+
+    want = oracle.dinic(g.n, g.off, g.dst, g.cap, g.s, g.t)
+    unpaired = back.copy()
+    unpaired[3] = 2 * g.m
+    for algo in (0, 1):
+        assert solve(back, algo) == 0 and flow.value == want
+        assert solve(unpaired, algo) == 1 and b"twin" in W.lib().wbpr_last_error()

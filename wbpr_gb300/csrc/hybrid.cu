@@ -488,7 +488,7 @@ __device__ void solve_hybrid(const ResParams& p, const HPart& P) {
 
 extern __shared__ __align__(16) char hyb_smem[];
 
-__global__ void __launch_bounds__(kResThreads) pr_hybrid(const __grid_constant__ ResParams p) {
+__global__ void __launch_bounds__(kResThreads, 1) pr_hybrid(const __grid_constant__ ResParams p) {
   HPart P;
   setup(p.in, p.rec, hyb_smem, P);
   build_records(p.in, P);
@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(kResThreads) pr_hybrid(const __grid_constant__
   solve_hybrid(p, P);
 }
 
-__global__ void __launch_bounds__(kResThreads) pr_hybrid_batch(const __grid_constant__ ResBatch b) {
+__global__ void __launch_bounds__(kResThreads, 1) pr_hybrid_batch(const __grid_constant__ ResBatch b) {
   ResParams p;
   int4* rec = b.rec + b.rec_stride * (blockIdx.x / cl_size());
   while (claim<true>(b, hyb_smem, p, rec)) {

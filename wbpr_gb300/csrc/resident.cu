@@ -16,8 +16,8 @@
 //
 // Measured on GB300, solve time before (persistent kernel) and now:
 //   GENRMF 4x5 (80 vertices, one block)            1.00 -> 0.13 ms
-//   GENRMF 8x16 (1,024 vertices, one block), RCSR  7.69 -> 0.69 ms
-//   layered 11x37 (409 vertices, one block), RCSR  1.91 -> 0.16 ms
+//   GENRMF 8x16 (1,024 vertices, one block), RCSR  7.69 -> 0.58 ms
+//   layered 11x37 (409 vertices, one block), RCSR  1.91 -> 0.14 ms
 //   GENRMF 16x40 (10,240 vertices, cluster)        33.8 -> 3.74 ms
 //   layered 32x256 (8,194 vertices, cluster)       2.96 -> 0.53 ms
 //   R-MAT scale 13 (221k residual arcs, cluster)   0.70 -> 0.47 ms
@@ -43,9 +43,13 @@ namespace {
 // layered 32x256 0.85, 0.53, 0.5-0.8 ms.
 constexpr int kResBfsLevels = 8;
 // Global relabel once the rounds since the last one took this many sixteenths
-// of its time, and at least 8 rounds.  GENRMF 16x40 at 4, 8, 16: 9.2, 6.0,
-// 3.8 ms; the small graphs gain 0-10% from 8 to 16.
+// of its time, and at least 8 rounds.  In a cluster at 4, 8, 16, 24: GENRMF
+// 16x40 9.2, 6.0, 3.8, 3.6 ms, layered 32x256 0.85, 0.93, 0.53, 0.66, R-MAT
+// scale 13 0.40, 0.41, 0.48, 0.57.  In one block at 16, 24, 32, 48: GENRMF 8x16
+// 0.67, 0.59, 0.58, 0.63 ms, 10x20 1.63, 1.52, 1.45, 1.56, layered 20x100
+// 0.34, 0.33, 0.31, 0.29.
 constexpr int kResGrShare = 16;
+constexpr int kResGrShareBlock = 28;
 
 // The layout of one block's memory and its share of the graph.  The vertices
 // are dealt to the groups of 32 slots (a warp looks after a group) in turn, and
@@ -517,7 +521,8 @@ __device__ void solve_resident(const ResParams& p, Part& P) {
 extern __shared__ __align__(16) char res_smem[];
 
 template <int W, bool CL>
-__global__ void __launch_bounds__(kResThreads) pr_resident(const __grid_constant__ ResParams p) {
+__global__ void __launch_bounds__(kResThreads, 1) pr_resident(const __grid_constant__ ResParams p) {
+  if (p.gate && (__ldcg(p.gate) | __ldcg(p.gate + 1) | __ldcg(p.gate + 2) | __ldcg(p.gate + 3))) return;
   Part P;
   if (!setup<CL>(p.in, res_smem, P)) {
     if (P.rank == 0 && threadIdx.x == 0) p.to.out->err = kResNoFit;
@@ -527,7 +532,7 @@ __global__ void __launch_bounds__(kResThreads) pr_resident(const __grid_constant
   solve_resident<W, CL>(p, P);
 }
 
-__global__ void __launch_bounds__(kResThreads) pr_resident_batch(const __grid_constant__ ResBatch b) {
+__global__ void __launch_bounds__(kResThreads, 1) pr_resident_batch(const __grid_constant__ ResBatch b) {
   ResParams p;
   while (claim<false>(b, res_smem, p, nullptr)) {
     Part P;
@@ -554,7 +559,7 @@ int resident_cluster(long long n, long long na) {
 cudaError_t launch_resident(const ResParams& p0, int tile, int cluster, cudaStream_t st) {
   ResParams p = p0;
     p.run.bsub = cluster == 1 ? 1 : kResBfsLevels;
-  p.run.grp = kResGrShare;
+  p.run.grp = cluster == 1 ? kResGrShareBlock : kResGrShare;
   if (cluster == 1) return tile < 32 ? launch_cluster<pr_resident<8, false>>(p, 1, st) : launch_cluster<pr_resident<32, false>>(p, 1, st);
   return tile < 32 ? launch_cluster<pr_resident<8, true>>(p, cluster, st) : launch_cluster<pr_resident<32, true>>(p, cluster, st);
 }
@@ -568,7 +573,7 @@ bool resident_one_block(long long n, long long na) {
 cudaError_t launch_resident_batch(const ResBatch& b0, int blocks, cudaStream_t st) {
   ResBatch b = b0;
   b.run.bsub = 1;
-  b.run.grp = kResGrShare;
+  b.run.grp = kResGrShareBlock;
   return launch_cluster<pr_resident_batch>(b, 1, st, blocks);
 }
 

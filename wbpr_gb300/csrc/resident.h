@@ -66,6 +66,7 @@ struct ResParams {
   ResInstance in;
   ResReport to;
   ResRun run;
+  const int* gate;  // nullptr, or four words that must all be 0: otherwise the launch does nothing
   bool keep;     // write residuals, labels and excess back
   int4* rec;     // hybrid only: one record a residual arc (hybrid.cu)
 };
