@@ -170,6 +170,7 @@ struct wbpr_graph {
   // unit-capacity bipartite shape of the terminal pair (mt_s, mt_t), and the
   // matching kernel's arrays (allocated at the first check)
   int mt_s = -1, mt_t = -1;
+  int64_t max_cap = -1;  // largest capacity, -1 unknown: a matching network's is 1
   bool mt_ok = false;
   int mt_nl = 0, mt_nl_light = 0, mt_nr = 0;
   long long mt_larcs = 0;
@@ -1322,7 +1323,7 @@ wbpr_status build_device(wbpr_graph* g, const wbpr_csr* in) {
   DB(cudaGetLastError());
   for (int k = 0; k < 3; ++k) DBS(device_scan(fl[k], (long long)n + 1, st));
   int tot[3];
-  unsigned long long hc[3];
+  unsigned long long hc[4];
   for (int k = 0; k < 3; ++k) DB(cudaMemcpyAsync(tot + k, fl[k] + n, 4, cudaMemcpyDeviceToHost, st));
   DB(cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
   DB(cudaMemcpyAsync(chk, cnt + 6, 16, cudaMemcpyDeviceToHost, st));
@@ -1340,6 +1341,7 @@ wbpr_status build_device(wbpr_graph* g, const wbpr_csr* in) {
   g->n_heavy = tot[2];
   g->n_td_heavy = (int)hc[0];
   g->n_td_items = (int64_t)hc[1];
+  g->max_cap = (int64_t)hc[3];
   g->total_deg = 2 * m;
   g->avg_deg = (double)g->total_deg / std::max<int64_t>(1, g->n_light + g->n_medium + g->n_heavy);
   DBS(dalloc(g, &g->cls, (size_t)(tot[0] + tot[1] + tot[2])));
@@ -1371,6 +1373,179 @@ wbpr_status build_device(wbpr_graph* g, const wbpr_csr* in) {
 }
 
 // ---------------------------------------------------------------------------
+// The per-vertex scratch of a handle, in one allocation of this many arrays.
+constexpr int kVertexArrays = 15;
+void vertex_arrays(wbpr_graph* g, int* base, size_t stride) {
+  int** vec[kVertexArrays] = {&g->h, &g->e, &g->rl_min, &g->rl_left, &g->lq[0], &g->lq[1], &g->hq[0], &g->hq[1],
+                              &g->esnap, &g->dmin0, &g->qraw, &g->fr[0], &g->fr[1], &g->fr[2], &g->vlab};
+  for (int k = 0; k < kVertexArrays; ++k) *vec[k] = base + k * stride;
+}
+
+// Graphs of at most this many arcs are built by the host: one copy to the
+// device instead of about 40 launches.  Measured on GB300, create of GENRMF 4x5
+// (304 arcs) 288 -> 55 us, 8x16 (4,544) 315 -> 94 us, 10x25 (11,400) 332 ->
+// 154 us, on RCSR 277 -> 49, 301 -> 86, 323 -> 135 us (16,000 arcs would be 10
+// ns each; the device build of 41,000 takes 363 us).
+constexpr int64_t kHostBuildArcs = 20000;
+
+// Everything a handle of a small graph holds, in one allocation: the arrays
+// the build fills (as the device build does, entry for entry), sent in one
+// copy, then the scratch.
+wbpr_status build_host(wbpr_graph* g, const wbpr_csr* in) {
+  NvtxRange nvtx_("host build");
+  wbpr_status st = wbpr::check_csr(in);
+  if (st) return st;
+  if (wbpr::max_in_capacity(in) > std::numeric_limits<int32_t>::max()) return WBPR_ERR_OVERFLOW;
+  const int n = g->n;
+  const size_t m = (size_t)g->m;
+  const bool bcsr = g->layout == WBPR_LAYOUT_BCSR;
+  wbpr::Bcsr16 rb;
+  wbpr::Rcsr rr;
+  if ((st = bcsr ? wbpr::build_bcsr16(in, &rb) : wbpr::build_rcsr_dev(in, &rr))) return st;
+  // length classes, long-row chunks and the sizes of the frontier and deep lists
+  auto length = [&](int u, int k) {
+    if (bcsr) return k ? 0 : rb.row[u + 1] - rb.row[u];
+    return k ? rr.rrow[u + 1] - rr.rrow[u] : rr.frow[u + 1] - rr.frow[u];
+  };
+  std::vector<int> cls[3];
+  size_t deep = 0;
+  g->n_td_items = 0;
+  for (int u = 0; u < n; ++u) {
+    const int d = length(u, 0) + length(u, 1);
+    if (d > 0) cls[d <= kLightDeg ? 0 : (d <= kHeavyDeg ? 1 : 2)].push_back(u);
+    if (d > kFirst) deep += (size_t)((d - kFirst + kPart - 1) / kPart);
+    if (d > kTdHeavy) {
+      ++g->n_td_heavy;
+      g->n_td_items += (d + kTdChunk - 1) / kTdChunk;
+    }
+  }
+  g->n_light = (int)cls[0].size();
+  g->n_medium = (int)cls[1].size();
+  g->n_heavy = (int)cls[2].size();
+  g->total_deg = 2 * g->m;
+  g->avg_deg = (double)g->total_deg / std::max<int64_t>(1, g->n_light + g->n_medium + g->n_heavy);
+  std::vector<int4> bch;
+  for (int u : cls[2])
+    for (int k = 0; k < 2; ++k) {
+      const int b = length(u, k) ? (bcsr ? rb.row[u] : (k ? rr.rrow[u] : rr.frow[u])) : 0, e = b + length(u, k);
+      for (int a = b; a < e; a += kChunk) bch.push_back(make_int4(u, k, a, std::min(e, a + kChunk)));
+    }
+  g->n_bch = (int)bch.size();
+  cls[0].insert(cls[0].end(), cls[1].begin(), cls[1].end());
+  cls[0].insert(cls[0].end(), cls[2].begin(), cls[2].end());
+  g->max_cap = 0;
+  for (size_t i = 0; i < m; ++i) g->max_cap = std::max<int64_t>(g->max_cap, in->capacities ? in->capacities[i] : 1);
+  // lay the memory out: filled arrays first
+  size_t at = 0;
+  auto room = [&](size_t bytes) {
+    const size_t here = at;
+    at = (at + std::max<size_t>(bytes, 16) + 255) & ~(size_t)255;
+    return here;
+  };
+  std::vector<char> host;
+  struct Fill {
+    const void* from;
+    size_t bytes, to;
+  };
+  std::vector<Fill> fills;
+  auto fill = [&](const void* from, size_t bytes) {
+    fills.push_back({from, bytes, room(bytes)});
+    return fills.back().to;
+  };
+  std::vector<int> zero(std::max<size_t>(m, (size_t)kLogSlots * kLogStride), 0);
+  const size_t rows = 4 * ((size_t)n + 1);
+  const size_t o_ioff = fill(in->offsets, rows), o_cls = fill(cls[0].data(), 4 * cls[0].size());
+  const size_t o_bch = fill(bch.data(), sizeof(int4) * bch.size());
+  size_t o_a, o_b, o_c, o_d = 0, o_e = 0, o_f = 0;
+  if (bcsr) {
+    o_a = fill(rb.row.data(), rows);
+    o_b = fill(rb.arc.data(), 16 * m);
+    o_c = fill(rb.arx.data(), 16 * m);
+    o_d = fill(zero.data(), sizeof(int) * (size_t)kLogSlots * kLogStride);
+  } else {
+    o_a = fill(rr.frow.data(), rows);
+    o_b = fill(rr.farc.data(), 8 * m);
+    o_c = fill(rr.fcap.data(), 4 * m);
+    o_d = fill(rr.rrow.data(), rows);
+    o_e = fill(rr.rarc.data(), 8 * m);
+    o_f = fill(zero.data(), 4 * m);
+  }
+  const size_t stride = ((size_t)n + 63) & ~(size_t)63;
+  const size_t o_vec = room(4 * stride * kVertexArrays);  // h and e, the first two, start as zeros
+  const size_t sent = o_vec + 8 * stride;
+  const size_t fstride = ((size_t)g->n_td_items + 1 + 31) & ~(size_t)31;
+  const size_t o_frh = room(3 * 8 * fstride), o_hrec = room(3 * 16 * (deep + 1)), o_hsum = room(4 * (deep + 1)),
+               o_hmin = room(4 * (deep + 1)), o_ctl = room(sizeof(Ctl)), o_st = room(sizeof(Stats)),
+               o_res = room(sizeof(ResOut));
+  const int64_t log = std::max<int64_t>(g->m / 2, (int64_t)1 << 20);
+  const size_t o_log = bcsr && m ? room(4 * (size_t)((log + kLogSlots - 1) / kLogSlots) * kLogSlots) : 0;
+  host.assign(sent, 0);
+  for (const Fill& f : fills)
+    if (f.bytes) std::memcpy(host.data() + f.to, f.from, f.bytes);
+  char* base = nullptr;
+  if ((st = dalloc(g, &base, at))) return st;
+  CK(cudaMemcpyAsync(base, host.data(), sent, cudaMemcpyHostToDevice, g->stream));
+  g->ioff = (int*)(base + o_ioff);
+  g->cls = (int*)(base + o_cls);
+  g->bch = (int4*)(base + o_bch);
+  if (bcsr) {
+    g->row = (int*)(base + o_a);
+    g->arc = (int2*)(base + o_b);
+    g->arx = (int2*)(base + o_c);
+    if (m) {
+      g->ulog_n = (int*)(base + o_d);
+      g->ulog = (int*)(base + o_log);
+      g->ulog_cap = (int)((log + kLogSlots - 1) / kLogSlots);
+    }
+  } else {
+    g->frow = (int*)(base + o_a);
+    g->farc = (int2*)(base + o_b);
+    g->fcap = (int*)(base + o_c);
+    g->rrow = (int*)(base + o_d);
+    g->rarc = (int2*)(base + o_e);
+    g->fcb = (int*)(base + o_f);
+  }
+  vertex_arrays(g, (int*)(base + o_vec), stride);
+  for (int k = 0; k < 3; ++k) g->frh[k] = (int2*)(base + o_frh) + k * fstride;
+  g->hrec = (int4*)(base + o_hrec);
+  g->hsum = (int*)(base + o_hsum);
+  g->hmin = (int*)(base + o_hmin);
+  g->ctl = (Ctl*)(base + o_ctl);
+  g->st = (Stats*)(base + o_st);
+  g->res_out = (ResOut*)(base + o_res);
+  CK(cudaStreamSynchronize(g->stream));
+  return WBPR_OK;
+}
+
+// The rest of a handle that the device built.
+wbpr_status build_on_device(wbpr_graph* g, const wbpr_csr* in) {
+  wbpr_status st = build_device(g, in);
+  if (st) return st;
+  const size_t stride = ((size_t)g->n + 63) & ~(size_t)63;
+  int* base = nullptr;
+  if ((st = dalloc(g, &base, stride * kVertexArrays))) return st;
+  vertex_arrays(g, base, stride);
+  const size_t fstride = ((size_t)g->n_td_items + 1 + 31) & ~(size_t)31;
+  int2* fb = nullptr;
+  if ((st = dalloc(g, &fb, 3 * fstride))) return st;
+  for (int k = 0; k < 3; ++k) g->frh[k] = fb + k * fstride;
+  if ((st = dalloc(g, &g->ctl, 1)) || (st = dalloc(g, &g->st, 1)) || (st = dalloc(g, &g->res_out, 1))) return st;
+  if (g->layout == WBPR_LAYOUT_BCSR && g->m > 0) {
+    // undo log: a quarter of the residual arcs (at least 2^20 entries), over
+    // kLogSlots slots; the built residuals are the capacities, so it starts empty
+    const int64_t want = std::max<int64_t>((2 * g->m) / 4, (int64_t)1 << 20);
+    g->ulog_cap = (int)((want + kLogSlots - 1) / kLogSlots);
+    if ((st = dalloc(g, &g->ulog, (size_t)g->ulog_cap * kLogSlots))) return st;
+    if ((st = dalloc(g, &g->ulog_n, (size_t)kLogSlots * kLogStride))) return st;
+    CK(cudaMemsetAsync(g->ulog_n, 0, sizeof(int) * (size_t)kLogSlots * kLogStride, g->stream));
+  }
+  // in the stream the pool allocations were made on (stream-ordered memory)
+  CK(cudaMemsetAsync(g->h, 0, 4 * (size_t)g->n, g->stream));
+  CK(cudaMemsetAsync(g->e, 0, 4 * (size_t)g->n, g->stream));
+  CK(cudaStreamSynchronize(g->stream));
+  return WBPR_OK;
+}
+
 wbpr_status create_impl(const wbpr_csr* in, wbpr_layout layout, wbpr_graph** out) {
   if (!out) return WBPR_ERR_INVALID_ARG;
   *out = nullptr;
@@ -1419,42 +1594,11 @@ wbpr_status create_impl(const wbpr_csr* in, wbpr_layout layout, wbpr_graph** out
   TRYC(cudaEventCreate(&g->ev1));
   TRYC(cudaEventCreate(&g->ev2));
   TRYC(cudaEventCreate(&g->ev3));
-  const int n = g->n;
-  TRY(build_device(g, in));
+  TRY(g->m <= kHostBuildArcs && g->n <= kHostBuildArcs ? build_host(g, in) : build_on_device(g, in));
   g->res_cluster = resident_cluster(g->n, g->total_deg);
   g->hybrid = hybrid_takes(g->n, g->total_deg, g->n_medium + g->n_heavy);
   // both could: see kResPreferUnits
   if (g->res_cluster > 1 && g->hybrid && g->n + g->total_deg > kResPreferUnits) g->res_cluster = 0;
-  int** vec[] = {&g->h, &g->e, &g->rl_min, &g->rl_left, &g->lq[0], &g->lq[1], &g->hq[0], &g->hq[1],
-                 &g->esnap, &g->dmin0,
-                 &g->qraw, &g->fr[0], &g->fr[1], &g->fr[2], &g->vlab};
-  {
-    // one allocation for the per-vertex scratch, one for the BFS chunk lists
-    const size_t nvec = sizeof(vec) / sizeof(vec[0]);
-    const size_t stride = ((size_t)n + 63) & ~(size_t)63;
-    int* base = nullptr;
-    TRY(dalloc(g, &base, stride * nvec));
-    for (size_t k = 0; k < nvec; ++k) *vec[k] = base + k * stride;
-    const size_t fstride = ((size_t)g->n_td_items + 1 + 31) & ~(size_t)31;
-    int2* fb = nullptr;
-    TRY(dalloc(g, &fb, 3 * fstride));
-    for (int k = 0; k < 3; ++k) g->frh[k] = fb + k * fstride;
-  }
-  TRY(dalloc(g, &g->ctl, 1));
-  TRY(dalloc(g, &g->st, 1));
-  if (g->layout == WBPR_LAYOUT_BCSR && g->m > 0) {
-    // undo log: a quarter of the residual arcs (at least 2^20 entries), over
-    // kLogSlots slots; the built residuals are the capacities, so it starts empty
-    const int64_t want = std::max<int64_t>((2 * g->m) / 4, (int64_t)1 << 20);
-    g->ulog_cap = (int)((want + kLogSlots - 1) / kLogSlots);
-    TRY(dalloc(g, &g->ulog, (size_t)g->ulog_cap * kLogSlots));
-    TRY(dalloc(g, &g->ulog_n, (size_t)kLogSlots * kLogStride));
-    TRYC(cudaMemsetAsync(g->ulog_n, 0, sizeof(int) * (size_t)kLogSlots * kLogStride, g->stream));
-  }
-  // in the stream the pool allocations were made on (stream-ordered memory)
-  TRYC(cudaMemsetAsync(g->h, 0, 4 * (size_t)n, g->stream));
-  TRYC(cudaMemsetAsync(g->e, 0, 4 * (size_t)n, g->stream));
-  TRYC(cudaStreamSynchronize(g->stream));
 #undef TRY
 #undef TRYC
   *out = g;
@@ -1646,10 +1790,6 @@ bool use_resident(const wbpr_graph* g, const RunCfg& rc) {
 // device without such clusters); nothing has changed then.
 wbpr_status run_resident(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch_ms, int* flow, bool* fits) {
   *fits = true;
-  if (!g->res_out) {
-    wbpr_status st = dalloc(g, &g->res_out, 1);
-    if (st) return st;
-  }
   ResInstance in{};
   in.n = g->n;
   in.mode = rc.mode;
@@ -2147,6 +2287,7 @@ wbpr_status wbpr_graph_set_capacities(wbpr_graph* g, const int32_t* capacities) 
                                                 dcap, g->n, g->m, 1, incap, chk);
   g->full_reset = true;  // every residual goes back to its new capacity at the next solve
   g->mt_s = g->mt_t = -1;  // capacities other than 1 may have come
+  g->max_cap = -1;
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(g->stream));
   return WBPR_OK;
@@ -2211,7 +2352,7 @@ wbpr_status wbpr_solve(wbpr_graph* g, int32_t s, int32_t t, wbpr_algo algo, cons
   rc.bfs_excl = s;
   CK(cudaSetDevice(g->device));
   bool matched = false;
-  if (rc.matching && (st = match_detect(g, s, t, &matched))) return st;
+  if (rc.matching && g->max_cap <= 1 && (st = match_detect(g, s, t, &matched))) return st;
   CK(cudaEventRecord(g->ev0, g->stream));
   Stats hs;
   float launch_ms = 0;
