@@ -65,7 +65,7 @@ struct Part {
   unsigned a0, a_rec, a_ve;  // shared-memory addresses: of the block's memory, of rec, of ve
   int cs, rank;
   unsigned a_row, a_ex;    // of row and ex
-  bool big;                // some row of this block is longer than a tile should walk
+  bool big;                // some row of this block is longer than kBigRow
   int groups;              // of 32 slots, the same in every block
   int nv, na;              // vertices and arcs of this block
   int n;                   // of the instance
@@ -168,12 +168,30 @@ __device__ bool setup(const ResInstance& in, char* sm, Part& P) {
   return true;
 }
 
-// Rows longer than this are walked by a whole warp.
-template <int W>
-__host__ __device__ constexpr unsigned big_row() { return W == 32 ? 0xffffffffu : W * 16u; }
+constexpr unsigned kBigRow = 128;  // rows longer than this are walked by a whole warp
+
+// Calls f(row j of the block, k) for the RCSR entries k of every row, forward
+// arcs first: 8 lanes a row, a warp for a long one (with 8 lanes there, R-MAT
+// scale 12 spent 0.13 ms of its 0.40 on loading its longest rows).
+template <class F>
+__device__ __forceinline__ void for_rows(const Part& P, F f) {
+  for (int j = threadIdx.x >> 3; j < P.nv; j += blockDim.x >> 3) {
+    const unsigned d = P.row[P.slot(j)] >> 16;
+    if (d <= kBigRow)
+      for (unsigned k = threadIdx.x & 7; k < d; k += 8) f(j, (int)k);
+  }
+  if (!P.big) return;
+  for (int j = threadIdx.x >> 5; j < P.nv; j += blockDim.x >> 5) {
+    const unsigned d = P.row[P.slot(j)] >> 16;
+    if (d > kBigRow) {
+#pragma unroll 4
+      for (unsigned k = threadIdx.x & 31; k < d; k += 32) f(j, (int)k);
+    }
+  }
+}
 
 // Reads this block's rows (residuals from the capacities in a fresh solve).
-template <int W, bool CL>
+template <bool CL>
 __device__ void load(const ResInstance& in, Part& P) {
   const ResCtl* c = P.c;
   const int v0 = c->bnd[P.rank], a0 = c->abase[P.rank];
@@ -187,7 +205,7 @@ __device__ void load(const ResInstance& in, Part& P) {
     if (i >= P.nv) continue;
     const int b = row_at(in, v0 + i) - a0, e = row_at(in, v0 + i + 1) - a0;
     P.row[k] = (unsigned)b | (unsigned)(e - b) << 16;
-    big |= (unsigned)(e - b) > big_row<W>();
+    big |= (unsigned)(e - b) > kBigRow;
     if (in.mode == kModeState) P.ve[k].y = __ldcg(in.e + in.vbase + v0 + i);
   }
   P.big = __syncthreads_or(big);
@@ -202,25 +220,23 @@ __device__ void load(const ResInstance& in, Part& P) {
     return;
   }
   Sh<CL>::sync();  // every block's memory may be written from here on
-  const int sub = threadIdx.x & 7, tile = threadIdx.x >> 3, nt = blockDim.x >> 3;
-  for (int i = tile; i < P.nv; i += nt) {
-    const int v = v0 + i;
-    const int fb = __ldg(in.frow + v), fe = __ldg(in.frow + v + 1), rb = __ldg(in.rrow + v), re = __ldg(in.rrow + v + 1);
-    for (int f = fb + sub; f < fe; f += 8) {
-      const int2 r = __ldcg(in.farc + f);
+  for_rows(P, [&](int j, int k) {
+    const int v = v0 + j, fb = __ldg(in.frow + v), nf = __ldg(in.frow + v + 1) - fb;
+    const int here = (int)(P.row[P.slot(j)] & 0xffff) + k;
+    int2* q = P.rec + here;
+    if (k < nf) {
+      const int2 r = __ldcg(in.farc + fb + k);
       const int o = owner_of(c, P.cs, r.x);
-      int2* q = P.rec + (f + rb - a0);
-      q->x = fresh ? __ldg(in.fcap + f) : r.y;
+      q->x = fresh ? __ldg(in.fcap + fb + k) : r.y;
       *(unsigned short*)&q->y = (unsigned short)(o << 12 | P.slot(r.x - c->bnd[o]));  // its twin is written below
-    }
-    for (int k = rb + sub; k < re; k += 8) {
-      const int2 r = __ldg(in.rarc + k);  // {tail, forward arc}
+    } else {
+      const int2 r = __ldg(in.rarc + __ldg(in.rrow + v) + k - nf);  // {tail, forward arc}
       const int o = owner_of(c, P.cs, r.x);
-      const int here = fe + k - a0, tw = r.y + __ldg(in.rrow + r.x) - c->abase[o];
-      P.rec[here] = make_int2(fresh ? 0 : __ldcg(in.fcb + r.y), (int)((unsigned)(o << 12 | P.slot(r.x - c->bnd[o])) | (unsigned)tw << 16));
+      const int tw = r.y + __ldg(in.rrow + r.x) - c->abase[o];
+      *q = make_int2(fresh ? 0 : __ldcg(in.fcb + r.y), (int)((unsigned)(o << 12 | P.slot(r.x - c->bnd[o])) | (unsigned)tw << 16));
       Sh<CL>::st16(Sh<CL>::at(P.a0, o) + P.a_rec + 8 * tw + 6, (unsigned)here);
     }
-  }
+  });
   Sh<CL>::sync();
 }
 
@@ -237,16 +253,13 @@ __device__ void write_back(const ResInstance& in, const Part& P) {
     for (int a = threadIdx.x; a < P.na; a += blockDim.x) in.arc[a0 + a].y = P.rec[a].x;
     return;
   }
-  const int sub = threadIdx.x & 7, tile = threadIdx.x >> 3, nt = blockDim.x >> 3;
-  for (int i = tile; i < P.nv; i += nt) {
-    const int v = v0 + i;
-    const int fb = __ldg(in.frow + v), fe = __ldg(in.frow + v + 1), rb = __ldg(in.rrow + v);
-    for (int f = fb + sub; f < fe; f += 8) {
-      const int cf = P.rec[f + rb - a0].x;
-      in.farc[f].y = cf;
-      in.fcb[f] = __ldg(in.fcap + f) - cf;
-    }
-  }
+  for_rows(P, [&](int j, int k) {
+    const int f = __ldg(in.frow + v0 + j) + k;
+    if (f >= __ldg(in.frow + v0 + j + 1)) return;
+    const int cf = P.rec[(P.row[P.slot(j)] & 0xffff) + k].x;
+    in.farc[f].y = cf;
+    in.fcb[f] = __ldg(in.fcap + f) - cf;
+  });
 }
 
 // Expands the vertices in slots u (one per W-lane tile, -1 for none) of label
@@ -293,7 +306,7 @@ __device__ int bfs_resident(const ResParams& p, Part& P, int& seq, Count& ct) {
         now = true;
         if (open) P.ex[i] = (unsigned short)l;
         if (W < 32 && P.big) {
-          unsigned big = __ballot_sync(kFull, open && P.row[i] >> 16 > big_row<W>());
+          unsigned big = __ballot_sync(kFull, open && P.row[i] >> 16 > kBigRow);
           mask &= ~big;
           for (; big; big &= big - 1) {
             const int t = __ffs(big) - 1;
@@ -423,7 +436,7 @@ __device__ __forceinline__ bool push_step(const Part& P, Count& ct) {
     if (!mask) continue;
     did = true;
     if (W < 32 && P.big) {
-      unsigned big = __ballot_sync(kFull, act && P.row[i] >> 16 > big_row<W>());
+      unsigned big = __ballot_sync(kFull, act && P.row[i] >> 16 > kBigRow);
       mask &= ~big;
       for (; big; big &= big - 1) discharge<32, CL>(P, g * 32 + __ffs(big) - 1, ct);
     }
@@ -528,7 +541,7 @@ __global__ void __launch_bounds__(kResThreads, 1) pr_resident(const __grid_const
     if (P.rank == 0 && threadIdx.x == 0) p.to.out->err = kResNoFit;
     return;
   }
-  load<W, CL>(p.in, P);
+  load<CL>(p.in, P);
   solve_resident<W, CL>(p, P);
 }
 
@@ -540,7 +553,7 @@ __global__ void __launch_bounds__(kResThreads, 1) pr_resident_batch(const __grid
       if (threadIdx.x == 0) *p.to.flow = -1;
       continue;
     }
-    load<8, false>(p.in, P);
+    load<false>(p.in, P);
     solve_resident<8, false>(p, P);
   }
 }
