@@ -963,7 +963,7 @@ __device__ __forceinline__ int seg_len(const int* o, int u) { return o ? __ldg(o
 // length classes (flags for three stable compactions) and the chunk counts
 // cnt: [0] rows > kTdHeavy [1] their top-down chunk items [2] bound on the deep
 // parts of a push phase (every vertex is filed at most once a round)
-__global__ void db_classify(const int* o1, const int* o2, int n, int* f0, int* f1, int* f2,
+__global__ void db_classify(const int* o1, const int* o2, int n, int first, int* f0, int* f1, int* f2,
                             unsigned long long* cnt) {
   unsigned long long a = 0, b = 0, c = 0;
   for (int u = blockIdx.x * blockDim.x + threadIdx.x; u <= n; u += gridDim.x * blockDim.x) {
@@ -971,7 +971,7 @@ __global__ void db_classify(const int* o1, const int* o2, int n, int* f0, int* f
     f0[u] = d > 0 && d <= kLightDeg;
     f1[u] = d > kLightDeg && d <= kHeavyDeg;
     f2[u] = d > kHeavyDeg;
-    if (d > kFirst) c += (d - kFirst + kPart - 1) / kPart;  // deep parts of the row
+    if (d > first) c += (d - first + kPart - 1) / kPart;  // deep parts of the row
     if (d > kTdHeavy) {
       a += 1;
       b += (d + kTdChunk - 1) / kTdChunk;
@@ -1319,7 +1319,7 @@ wbpr_status build_device(wbpr_graph* g, const wbpr_csr* in) {
   const int* o2 = bcsr ? nullptr : g->rrow;
   // length classes in vertex order, by three stable compactions
   int* fl[3] = {vb[0], vb[1], kb[0]};  // free once the fill kernels have run (stream order)
-  db_classify<<<blocks, 256, 0, st>>>(o1, o2, n, fl[0], fl[1], fl[2], cnt);
+  db_classify<<<blocks, 256, 0, st>>>(o1, o2, n, first_arcs(n + 2 * m), fl[0], fl[1], fl[2], cnt);
   DB(cudaGetLastError());
   for (int k = 0; k < 3; ++k) DBS(device_scan(fl[k], (long long)n + 1, st));
   int tot[3];
@@ -1408,12 +1408,13 @@ wbpr_status build_host(wbpr_graph* g, const wbpr_csr* in) {
     return k ? rr.rrow[u + 1] - rr.rrow[u] : rr.frow[u + 1] - rr.frow[u];
   };
   std::vector<int> cls[3];
+  const int first = first_arcs(n + 2 * g->m);
   size_t deep = 0;
   g->n_td_items = 0;
   for (int u = 0; u < n; ++u) {
     const int d = length(u, 0) + length(u, 1);
     if (d > 0) cls[d <= kLightDeg ? 0 : (d <= kHeavyDeg ? 1 : 2)].push_back(u);
-    if (d > kFirst) deep += (size_t)((d - kFirst + kPart - 1) / kPart);
+    if (d > first) deep += (size_t)((d - first + kPart - 1) / kPart);
     if (d > kTdHeavy) {
       ++g->n_td_heavy;
       g->n_td_items += (d + kTdChunk - 1) / kTdChunk;
@@ -1721,6 +1722,7 @@ wbpr_status run_kernel(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch
   p.t = rc.t;
   p.mode = rc.mode;
   p.heavy_deg = rc.heavy_deg;
+  p.first = first_arcs((long long)g->n + g->total_deg);
   p.gr_threshold = rc.gr_threshold;
   p.gr_rounds = rc.gr_rounds;
   p.gr_stall = rc.gr_stall;

@@ -9,7 +9,7 @@
 //
 // Limits: at most kNoAllocMaxVertices vertices and kNoAllocMaxArcs residual
 // arcs (two per input arc); larger graphs are refused with
-// WBPR_ERR_INVALID_ARG.  The array occupies about 5.6 MB on every device that
+// WBPR_ERR_INVALID_ARG.  The array occupies about 6 MB on every device that
 // loads the library, until the process exits.
 //
 // Set-up: the first call on a device (with that device current) looks up the
@@ -42,9 +42,10 @@ constexpr long long kStatWords = align_ints((sizeof(Stats) + 3) / 4);
 constexpr long long kCountWords = 64;  // classification counters
 constexpr int kVertexArrays = 15;      // per-vertex int arrays, indexed as in wbpr_solve_bcsr_noalloc
 constexpr long long kTdItems = kNoAllocMaxArcs / kTdChunk + kNoAllocMaxVertices;
-// deep parts: rows longer than kFirst, each filed at most once a round, cut
-// into kPart-arc parts beyond their first kFirst arcs
-constexpr long long kChunkItems = kNoAllocMaxArcs / kPart + kNoAllocMaxArcs / (kFirst + 1) + 1;
+// deep parts: rows longer than first_arcs() (256 at these sizes), each filed at
+// most once a round, cut into kPart-arc parts beyond their first 256 arcs
+static_assert(kNoAllocMaxVertices + kNoAllocMaxArcs <= kFirstUnits[0]);
+constexpr long long kChunkItems = align_ints(kNoAllocMaxArcs / kPart + kNoAllocMaxArcs / (256 + 1) + 1);
 constexpr long long kBchItems = kNoAllocMaxArcs / kChunk + kNoAllocMaxArcs / (kHeavyDeg + 1) + 1;
 constexpr long long kOffStat = kCtlWords;
 constexpr long long kOffCount = kOffStat + kStatWords;
@@ -52,6 +53,7 @@ constexpr long long kOffVert = kOffCount + kCountWords;
 constexpr long long kOffFrh = kOffVert + (long long)kVertexArrays * kNoAllocMaxVertices;
 constexpr long long kOffChunk = kOffFrh + 3 * 2 * kTdItems;
 constexpr long long kOffBch = kOffChunk + 14 * kChunkItems;  // hrec (3 x int4), hsum, hmin per item
+static_assert(kOffChunk % 4 == 0 && kOffBch % 4 == 0, "int4 arrays");
 constexpr long long kScratchWords = align_ints(kOffBch + 4 * kBchItems);
 
 static __device__ __align__(256) int g_noalloc_scratch[kScratchWords];
@@ -380,6 +382,7 @@ extern "C" wbpr_status wbpr_solve_bcsr_noalloc(int32_t n, int64_t num_residual_a
   p.budget_ns = 120ull * 1000 * 1000 * 1000;
   p.bar_timeout_ns = 10ull * 1000 * 1000 * 1000;
   p.heavy_deg = 32;
+  p.first = first_arcs((long long)n + num_residual_arcs);
   p.mode = kModeFresh;
   p.bfs_excl = s;
   const int tile = algo == WBPR_ALGO_TC ? 1 : 32;

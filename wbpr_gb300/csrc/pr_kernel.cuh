@@ -370,6 +370,7 @@ struct Params {
   unsigned long long budget_ns;
   unsigned long long bar_timeout_ns;
   int heavy_deg;
+  int first;     // arcs of a heavy row walked by one warp before it goes deep (first_arcs)
   int mode;
   int bfs_dir;   // 0: vertices that reach the root (to sink); 1: reached from the root
   int bfs_root;
@@ -551,14 +552,21 @@ __device__ __forceinline__ void vidx(const VRow& r, int vi, int& k, int& a) {
   }
 }
 
-// Long rows are walked by one warp over their first kFirst arcs; a vertex
+// Long rows are walked by one warp over their first `first` arcs; a vertex
 // that still has excess after them becomes a deep entry, and the rest of its
 // row is cut into kPart-arc parts that warps of the whole grid process in two
 // passes (deep passes A and B below).
-#ifndef WBPR_FIRST_ARCS
-#define WBPR_FIRST_ARCS 2048
-#endif
-constexpr int kFirst = WBPR_FIRST_ARCS;  // arcs of a long row walked by one warp before it goes deep
+//
+// A warp's walk is a chain of batches of 128 arcs, about 1.3 us each, so on
+// small graphs, where few rows are active, the longest walk is what the first
+// pass waits for; on the largest the deep passes, which read every part of a
+// row, cost more than it gives.  Measured on GB300 at 2,048, 1,024, 512 and 256
+// arcs, R-MAT on BCSR16: scale 17 1.37, 1.26, 1.19, 1.14 ms; 18 1.33, 1.22,
+// 1.13, 1.10; 20 2.47, 2.32, 2.17, 2.20; 21 2.70, 2.40, 2.33, 2.20; 22 3.63,
+// 3.69, 3.58, 3.63.  On RCSR: scale 17 1.64, 1.42, 1.30, 1.24; 20 2.52, 2.46,
+// 2.53, 2.48; 21 3.54, 2.95, 2.83, 2.89; 22 4.87, 6.78, 6.50, 6.38.
+constexpr long long kFirstUnits[2] = {1LL << 24, 100000000};  // n + residual arcs, for 256 and 512 arcs
+inline int first_arcs(long long units) { return units <= kFirstUnits[0] ? 256 : (units <= kFirstUnits[1] ? 512 : 2048); }
 constexpr int kPart = 256;               // arcs of a deep part: one warp, 8 arcs a lane in flight
 
 template <class Topo>
@@ -683,7 +691,7 @@ __device__ __forceinline__ void tile_discharge(const Params<Topo>& p, int u, int
 }
 
 // ---------------------------------------------------------------------------
-// Deep entries: the part of a long row beyond its first kFirst arcs, cut into
+// Deep entries: the part of a long row beyond its first `first` arcs, cut into
 // kPart-arc parts, each processed by one warp in two passes of the push phase:
 //   pass A  every part sums the residual capacity of its admissible arcs
 //           (saturated at the vertex's excess left) and takes the minimum
@@ -701,7 +709,7 @@ __device__ __forceinline__ void tile_discharge(const Params<Topo>& p, int u, int
 //
 // Part record (3 x int4, 48 bytes: all a warp needs, in one load):
 //   {u, first part of the entry, E (excess at filing), E left after the first
-//    kFirst arcs}, {label, parts, entry, first arc of part 0}, the row
+//    first arcs}, {label, parts, entry, first arc of part 0}, the row
 //   {b0, d0, b1, deg}.
 
 // Settle a vertex: subtract what it pushed, re-file it when it still has
@@ -861,7 +869,7 @@ __device__ void push_first(const Params<Topo>& p, int cur, int raw, BlockAcc& ac
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int idx = gw; idx < nH;) {
-    tile_discharge<Topo, 32, 4>(p, __ldcg(p.hq[cur] + idx), kFirst, rawcnt, acc);
+    tile_discharge<Topo, 32, 4>(p, __ldcg(p.hq[cur] + idx), p.first, rawcnt, acc);
     int nx = 0;
     if (lane == 0) nx = nwarps + atomicAdd(&c->heavy_next, 1);
     idx = __shfl_sync(0xffffffffu, nx, 0);
@@ -873,7 +881,7 @@ __device__ void push_first(const Params<Topo>& p, int cur, int raw, BlockAcc& ac
 #pragma unroll 1
     for (int r = 0; r < 2; ++r) {
       const int idx = base + r * kTpw + lane / W;
-      if (idx < nL) tile_discharge<Topo, W, 4>(p, __ldcg(p.lq[cur] + idx), kFirst, rawcnt, acc);
+      if (idx < nL) tile_discharge<Topo, W, 4>(p, __ldcg(p.lq[cur] + idx), kBig, rawcnt, acc);  // never deep
     }
     __syncwarp();
     int nx = 0;
