@@ -782,6 +782,7 @@ __global__ void __launch_bounds__(256, 4) db_sort_scatter(const int* kin, const 
   __shared__ int dstart[256];    // tile-local start of each digit
   __shared__ int gofs[256];      // global start of this tile's run of each digit
   __shared__ int sk[kSortTile], sv[kSortTile];
+  __shared__ int nvalid;  // arcs placed in sk and sv
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = threadIdx.x;
   const int tile = blockIdx.x;
   const unsigned lt = (1u << lane) - 1;
@@ -827,6 +828,7 @@ __global__ void __launch_bounds__(256, 4) db_sort_scatter(const int* kin, const 
   int wpre = 0;
   for (int j = 0; j < w; ++j) wpre += ws[j];
   dstart[t] = wpre + inc - tot;
+  if (t == 255) nvalid = wpre + inc;
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < kSortRounds; ++r) {
@@ -837,8 +839,10 @@ __global__ void __launch_bounds__(256, 4) db_sort_scatter(const int* kin, const 
     sv[lp] = val[r];
   }
   __syncthreads();
-  const int cnt = (int)min((long long)kSortTile, m - (long long)tile * kSortTile);
-  for (int i = t; i < cnt; i += 256) {
+  // only what the tile placed: a negative head (refused after the sort) is
+  // counted by the histogram but has no slot here, and the words past the
+  // placed ones would be written wherever their stale digits point
+  for (int i = t; i < nvalid; i += 256) {
     const int k = sk[i];
     const int d = (k >> shift) & 255;
     const int pos = gofs[d] + (i - dstart[d]);
