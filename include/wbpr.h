@@ -396,7 +396,7 @@ wbpr_status wbpr_batch_autotune(wbpr_batch* b, wbpr_tuning* best, float* best_ms
  * at num_residual_arcs and never decrease; heads must lie in [0, n), twins be
  * paired, capacities be >= 0 (WBPR_ERR_INVALID_ARG otherwise); and no vertex's
  * incoming capacities may sum past int32 (WBPR_ERR_OVERFLOW).  All solver
- * scratch lives in one fixed file-scope device array (about 5.6 MB per device,
+ * scratch lives in one fixed file-scope device array (about 6 MB per device,
  * held until exit), so no allocation happens.  Limits: n <= 65536 vertices and
  * num_residual_arcs <= 1048576; larger inputs return WBPR_ERR_INVALID_ARG (see
  * wbpr_last_error).  The first call on a device looks up the array's address;
