@@ -42,10 +42,10 @@ constexpr long long kStatWords = align_ints((sizeof(Stats) + 3) / 4);
 constexpr long long kCountWords = 64;  // classification counters
 constexpr int kVertexArrays = 15;      // per-vertex int arrays, indexed as in wbpr_solve_bcsr_noalloc
 constexpr long long kTdItems = kNoAllocMaxArcs / kTdChunk + kNoAllocMaxVertices;
-// deep parts: rows longer than first_arcs() (256 at these sizes), each filed at
-// most once a round, cut into kPart-arc parts beyond their first 256 arcs
+// deep parts: rows longer than first_arcs() (128 at these sizes), each filed at
+// most once a round, cut into kPart-arc parts beyond their first 128 arcs
 static_assert(kNoAllocMaxVertices + kNoAllocMaxArcs <= kFirstUnits[0]);
-constexpr long long kChunkItems = align_ints(kNoAllocMaxArcs / kPart + kNoAllocMaxArcs / (256 + 1) + 1);
+constexpr long long kChunkItems = align_ints(kNoAllocMaxArcs / kPart + kNoAllocMaxArcs / (128 + 1) + 1);
 constexpr long long kBchItems = kNoAllocMaxArcs / kChunk + kNoAllocMaxArcs / (kHeavyDeg + 1) + 1;
 constexpr long long kOffStat = kCtlWords;
 constexpr long long kOffCount = kOffStat + kStatWords;

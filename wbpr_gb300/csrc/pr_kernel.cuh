@@ -564,9 +564,14 @@ __device__ __forceinline__ void vidx(const VRow& r, int vi, int& k, int& a) {
 // arcs, R-MAT on BCSR16: scale 17 1.37, 1.26, 1.19, 1.14 ms; 18 1.33, 1.22,
 // 1.13, 1.10; 20 2.47, 2.32, 2.17, 2.20; 21 2.70, 2.40, 2.33, 2.20; 22 3.63,
 // 3.69, 3.58, 3.63.  On RCSR: scale 17 1.64, 1.42, 1.30, 1.24; 20 2.52, 2.46,
-// 2.53, 2.48; 21 3.54, 2.95, 2.83, 2.89; 22 4.87, 6.78, 6.50, 6.38.
-constexpr long long kFirstUnits[2] = {1LL << 24, 100000000};  // n + residual arcs, for 256 and 512 arcs
-inline int first_arcs(long long units) { return units <= kFirstUnits[0] ? 256 : (units <= kFirstUnits[1] ? 512 : 2048); }
+// 2.53, 2.48; 21 3.54, 2.95, 2.83, 2.89; 22 4.87, 6.78, 6.50, 6.38.  At 256 and
+// 128 arcs (one batch), means of three seeds: BCSR16 scale 15 0.85, 0.79 ms, 16
+// 1.03, 1.00, 17 (2.8M units) 1.07, 1.02, 18 (8.1M units) 1.05, 1.06; RCSR 0.91,
+// 0.88, 1.10, 1.08, 1.14, 1.09, 1.05, 1.07.
+constexpr long long kFirstUnits[3] = {1LL << 22, 1LL << 24, 100000000};  // n + residual arcs, for 128, 256 and 512 arcs
+inline int first_arcs(long long units) {
+  return units <= kFirstUnits[0] ? 128 : (units <= kFirstUnits[1] ? 256 : (units <= kFirstUnits[2] ? 512 : 2048));
+}
 constexpr int kPart = 256;               // arcs of a deep part: one warp, 8 arcs a lane in flight
 
 template <class Topo>
