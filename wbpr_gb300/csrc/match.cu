@@ -539,79 +539,6 @@ __device__ bool match_gr(const MatchParams& p, int qb, MAcc& acc, int& levels, i
   return true;
 }
 
-// The closure test.  Most active vertices that have lost their way to t sit in
-// tiny sets that are closed under pushes: a right vertex and the two or three
-// left ones that have no other neighbour (on the 2M x 2M matching the median
-// closure holds 2 left vertices, the largest of a sample 28).  A thread follows
-// its vertex's pushes -- neighbours, their mates, those mates' neighbours --
-// and when it comes to an end without a free right vertex within kClosure left
-// vertices, retires the whole set (label n, as a global relabel would).  A
-// global relabel reads every row that free right vertices reach instead: there
-// the second one took 0.42 ms to retire 400 vertices (the solve 1.87 -> 1.50
-// ms; with a test of 427,000 vertices before the first relabel 1.96 ms, 3 rounds
-// between tests 1.64, sets of 32 1.52).
-// Nothing else changes during the test, and sets that overlap are retired with
-// the same words.  The survivors become the active lists fr[0], fr[1] (counts
-// cq).  False when a barrier failed.
-constexpr int kClosure = 16;
-constexpr int kTestRounds = 6;    // rounds between two tests
-constexpr int kFewActive = 4096;  // active vertices that may wait for rounds instead of a relabel
-constexpr int kVeryFew = 64;      // too few to tell whether tests pay
-
-__device__ __forceinline__ bool closed(const MatchParams& p, int x, MAcc& acc) {
-  int set[kClosure];
-  int cnt = 1;
-  set[0] = x;
-  for (int i = 0; i < cnt; ++i) {
-    int b;
-    const int d = left_row(p, set[i], b);
-    if (d > p.heavy_deg) return false;
-    for (int k0 = 0; k0 < d; k0 += 4) {
-      int y[4];
-      unsigned long long w[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) y[j] = k0 + j < d ? __ldg(&p.lhd[b + k0 + j].x) : -1;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = y[j] >= 0 ? __ldcg(p.mate + y[j]) : mword((unsigned)x, 0);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int m = wmate(w[j]);
-        if (m < 0) return false;        // a free right vertex: x reaches t
-        if (y[j] >= 0) ++acc.bfs_arcs;
-        if (wlab(w[j]) >= p.n) continue;  // known to be dead
-        bool in = false;
-        for (int q = 0; q < cnt; ++q) in |= set[q] == m;
-        if (in) continue;
-        if (cnt == kClosure) return false;
-        set[cnt++] = m;
-      }
-    }
-  }
-  for (int i = 0; i < cnt; ++i) {
-    int b;
-    const int d = left_row(p, set[i], b);
-    p.lab[set[i]] = p.n;
-    for (int k = 0; k < d; ++k) {
-      const int y = __ldg(&p.lhd[b + k].x);
-      p.mate[y] = mword((unsigned)wmate(__ldcg(p.mate + y)), p.n);
-    }
-  }
-  return true;
-}
-
-__device__ bool match_closures(const MatchParams& p, const int* L, int nL, const int* H, int nH, MAcc& acc) {
-  MCtl* c = p.ctl;
-  const int gt = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
-  if (gt == 0) c->cq[0] = c->cq[1] = 0;
-  if (!grid_sync(c, p.bar_timeout_ns)) return false;
-  for (int i = gt; i < nL; i += gs) {
-    const int x = __ldcg(L + i);
-    if (!closed(p, x, acc)) append(p.fr[0], &c->cq[0], x);
-  }
-  for (int i = gt; i < nH; i += gs) append(p.fr[1], &c->cq[1], __ldcg(H + i));
-  return grid_sync(c, p.bar_timeout_ns);
-}
-
 // Four blocks of 256 per SM (64 registers): at three (80 registers, what the
 // compiler picks unbounded) the relabels' latency-bound levels ran 1.7 ms
 // instead of 0.9 on the 2M x 2M matching.
@@ -648,14 +575,10 @@ __global__ void __launch_bounds__(256, 4) pr_match(MatchParams p) {
   unsigned long long gr_end = t_start, gr_last = 0;  // global thread 0 only
   int act_hist[kMaxPlateau];  // active counts of the last gr_plateau rounds
   bool need_gr = false, done = false, stopped = false, first = true;
-  bool inl = false;   // the active lists are the closure test's survivors
-  int next_test = 0;  // first round that may run it
-  bool tests = true, paid = false;  // it is still worth running; it has retired a quarter of a set
   // the stop and time-balance words as read after the last round's barrier:
   // global thread 0 rewrites both during the next round, which it may enter
   // while another block is still deciding whether to run it
-  bool stop = false;
-  int gr_ok = 3;  // the rounds since the last relabel took 1: half its time, 2: its time, 3: twice its time
+  bool stop = false, gr_ok = true;
   int nL = p.nl_light, nH = p.nl - p.nl_light;  // the first round takes every left vertex
   for (;;) {
     if (need_gr) {
@@ -671,7 +594,6 @@ __global__ void __launch_bounds__(256, 4) pr_match(MatchParams p) {
         TRACE(p, kTrGrEnd, 0, nL, nH);
       }
       need_gr = false;
-      inl = false;
       work = 0;
       since_gr = 0;
     }
@@ -690,27 +612,9 @@ __global__ void __launch_bounds__(256, 4) pr_match(MatchParams p) {
     // retires it at once.  The counts are final at the barrier, so every
     // block takes the same branch.
     if (p.gr_plateau > 0 && since_gr >= p.gr_plateau &&
-        (long long)nact * 10 >= (long long)act_hist[since_gr % p.gr_plateau] * 9) {
-      // After the first relabel the closure test comes first.  Where one has
-      // paid, and few vertices are left, the relabel waits until the rounds
-      // since the last one took as long as it did, or twice as long, not half:
-      // they may well be done by then.  A test that retires less than a
-      // quarter of a set is the solve's last (on uniform random graphs the
-      // closed sets are large).
-      if (grs > 0 && tests && rounds >= next_test) {
-        const int b = rounds & 1;
-        if (!match_closures(p, p.q[b], nL, p.hq[b], nH, acc)) break;
-        inl = true;
-        nL = ldv(&c->cq[0]);
-        nH = ldv(&c->cq[1]);
-        next_test = rounds + kTestRounds;
-        if (nact > kVeryFew) tests = paid = (long long)(nL + nH) * 4 <= (long long)nact * 3;
-        if (nL + nH == 0) continue;
-      }
-      if (gr_ok > (grs > 0 && paid ? (nact <= kFewActive) + (nact <= kVeryFew) : 0)) {
-        need_gr = true;
-        continue;
-      }
+        (long long)nact * 10 >= (long long)act_hist[since_gr % p.gr_plateau] * 9 && gr_ok) {
+      need_gr = true;
+      continue;
     }
     if (p.gr_plateau > 0) act_hist[since_gr % p.gr_plateau] = nact;
     const unsigned long long t0 = gtime();
@@ -721,19 +625,17 @@ __global__ void __launch_bounds__(256, 4) pr_match(MatchParams p) {
       c->work[(rounds + 1) % 3] = 0;
     }
     const unsigned long long w0 = acc.scanned + acc.visits, tb = gtime();
-    match_round(p, inl ? p.fr[0] : (first ? p.lv : p.q[b]), nL,
-                inl ? p.fr[1] : (first ? p.lv + p.nl_light : p.hq[b]), nH, b ^ 1, (rounds + 1) % 3, acc);
-    inl = false;
+    match_round(p, first ? p.lv : p.q[b], nL, first ? p.lv + p.nl_light : p.hq[b], nH, b ^ 1, (rounds + 1) % 3,
+                acc);
     add_block((long long*)&c->work[rounds % 3], (long long)(acc.scanned + acc.visits - w0));
     TRACE_BLOCK(p, tb);
     if (gt == 0) {
       if ((p.max_rounds > 0 && rounds + 1 >= p.max_rounds) || time_past(t_start, p.budget_ns)) c->stop = 1;
-      const unsigned long long since = gtime() - gr_end;
-      c->gr_ok = (2 * since >= gr_last) + (since >= gr_last) + (since >= 2 * gr_last);
+      c->gr_ok = 2 * (gtime() - gr_end) >= gr_last;
     }
     if (!grid_sync(c, p.bar_timeout_ns)) break;
     stop = ldv(&c->stop) != 0;
-    gr_ok = ldv(&c->gr_ok);
+    gr_ok = ldv(&c->gr_ok) != 0;
     nL = ldv(&c->qn[(rounds + 1) % 3]);
     nH = ldv(&c->hn[(rounds + 1) % 3]);
     work += ldv64u(&c->work[rounds % 3]);

@@ -23,8 +23,6 @@ struct MCtl {
   alignas(128) int qn[3];     // light active queue counts, by round % 3
   alignas(128) int hn[3];     // heavy active queue counts, by round % 3
   alignas(128) int gq[2];     // the queue a global relabel builds: light, heavy
-  alignas(128) int cq[2];     // the closure test's survivors: light, heavy (not gq, which a relabel
-                              // right after the test clears while some block may still read)
   alignas(128) int fn[3];     // right vertices labelled by a BFS level, by level % 3
   alignas(128) int mcnt[2];   // materialised frontier lists
   alignas(128) long long fdeg[3];  // their reverse arcs
