@@ -1607,7 +1607,7 @@ wbpr_status create_impl(const wbpr_csr* in, wbpr_layout layout, wbpr_graph** out
   TRYC(cudaEventCreate(&g->ev3));
   TRY(g->m <= kHostBuildArcs && g->n <= kHostBuildArcs ? build_host(g, in) : build_on_device(g, in));
   g->res_cluster = resident_cluster(g->n, g->total_deg);
-  g->hybrid = hybrid_takes(g->n, g->total_deg, g->n_medium + g->n_heavy);
+  g->hybrid = g->n + g->total_deg <= kHybMaxUnits && hybrid_takes(g->n, g->total_deg, g->n_medium + g->n_heavy);
   // both could: see kResPreferUnits
   if (g->res_cluster > 1 && g->hybrid && g->n + g->total_deg > kResPreferUnits) g->res_cluster = 0;
 #undef TRY

@@ -100,16 +100,21 @@ __device__ __forceinline__ int4 record(const int4* rec, int a) {
   return v;
 }
 
-__device__ void setup(const ResInstance& in, int4* rec, char* sm, HPart& P) {
-  ResCtl* c = (ResCtl*)sm;
-  P.c = c;
-  P.cs = (int)cl_size();
-  P.rank = (int)cl_rank();
-  P.shift = 31 - __clz(P.cs);
+// How the vertices are dealt to a cluster of cs blocks.
+__device__ void shape(const ResInstance& in, int4* rec, int cs, HPart& P) {
+  P.cs = cs;
+  P.shift = 31 - __clz(cs);
   P.n = in.n;
   P.rec = rec;
   P.row0 = row_at(in, 0);
-  P.groups = max((int)blockDim.x >> 5, ((in.n + P.cs - 1) / P.cs + 127) >> 7);
+  P.groups = max(kResThreads >> 5, ((in.n + cs - 1) / cs + 127) >> 7);
+}
+
+__device__ void setup(const ResInstance& in, int4* rec, char* sm, HPart& P) {
+  ResCtl* c = (ResCtl*)sm;
+  P.c = c;
+  shape(in, rec, (int)cl_size(), P);
+  P.rank = (int)cl_rank();
   const unsigned slots = 128 * P.groups;
   P.a0 = sm_addr(sm);
   P.a_list = (sizeof(ResCtl) + 15) & ~15u;
@@ -148,10 +153,9 @@ __device__ __forceinline__ int2 row_of(const ResInstance& in, const HPart& P, in
   return make_int2(b - P.row0, row_at(in, v + 1) - b);
 }
 
-// Builds the records, every arc by the next thread of the cluster.
-__device__ void build_records(const ResInstance& in, const HPart& P) {
+// Builds the records, every arc by the next of nt threads.
+__device__ void build_records(const ResInstance& in, const HPart& P, int tid, int nt) {
   const bool fresh = in.mode == kModeFresh;
-  const int tid = P.rank * blockDim.x + threadIdx.x, nt = P.cs * blockDim.x;
   if (in.row) {
     const int na = row_at(in, in.n) - P.row0;
 #pragma unroll 4
@@ -186,8 +190,10 @@ __device__ void write_back(const ResInstance& in, const HPart& P) {
     in.lab[in.vbase + v] = (int)lds32(P.a0 + P.a_lab + 4 * i);
     if (in.mode != kModeBfsOnly) in.e[in.vbase + v] = (int)lds32(P.a0 + P.a_e + 4 * i);
   }
-  if (in.mode == kModeBfsOnly) return;
-  const int tid = P.rank * blockDim.x + threadIdx.x, nt = P.cs * blockDim.x;
+}
+
+// The residuals from the records, every arc by the next of nt threads.
+__device__ void write_arcs(const ResInstance& in, const HPart& P, int tid, int nt) {
   if (in.row) {
     const int na = row_at(in, in.n) - P.row0;
 #pragma unroll 4
@@ -488,10 +494,29 @@ __device__ void solve_hybrid(const ResParams& p, const HPart& P) {
 
 extern __shared__ __align__(16) char hyb_smem[];
 
+// A single solve's records are built, and its residuals written back, by the
+// whole GPU in launches of their own: the cluster's 16 SMs took longer over
+// them than over a solve of few rounds.  In the cluster and now, on RCSR (whose
+// records need a search for the row of each reverse entry) and BCSR16: random
+// graphs of 280,000 vertices with 1.7M arcs 1.81 -> 0.72 and 0.99 -> 0.66 ms,
+// with 0.4M 1.25 -> 0.81 and 1.04 -> 0.97; sink side of the cut of a 512x512
+// grid 1.07 -> 0.66 and 0.79 -> 0.64 ms.  Below 200,000 units nothing changes.
+// (In a batch the other SMs have instances of their own.)
+constexpr int kArcBlocks = 152 * 8;
+__global__ void __launch_bounds__(256) hybrid_load(const __grid_constant__ ResParams p) {
+  HPart P;
+  shape(p.in, p.rec, kResMaxCluster, P);
+  build_records(p.in, P, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+__global__ void __launch_bounds__(256) hybrid_store(const __grid_constant__ ResParams p) {
+  HPart P;
+  shape(p.in, p.rec, kResMaxCluster, P);
+  write_arcs(p.in, P, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
 __global__ void __launch_bounds__(kResThreads, 1) pr_hybrid(const __grid_constant__ ResParams p) {
   HPart P;
   setup(p.in, p.rec, hyb_smem, P);
-  build_records(p.in, P);
   Smem::sync();
   solve_hybrid(p, P);
 }
@@ -502,7 +527,7 @@ __global__ void __launch_bounds__(kResThreads, 1) pr_hybrid_batch(const __grid_c
   while (claim<true>(b, hyb_smem, p, rec)) {
     HPart P;
     setup(p.in, p.rec, hyb_smem, P);
-    build_records(p.in, P);
+    build_records(p.in, P, P.rank * blockDim.x + threadIdx.x, P.cs * blockDim.x);
     Smem::sync();
     solve_hybrid(p, P);
   }
@@ -514,7 +539,14 @@ cudaError_t launch_hybrid(const ResParams& p0, cudaStream_t st) {
   ResParams p = p0;
   p.run.bsub = kHybBfsLevels;
   p.run.grp = kHybGrShare;
-  return launch_cluster<pr_hybrid>(p, kResMaxCluster, st);
+  hybrid_load<<<kArcBlocks, 256, 0, st>>>(p);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = launch_cluster<pr_hybrid>(p, kResMaxCluster, st);
+  if (e == cudaSuccess && p.keep && p.in.mode != kModeBfsOnly) {
+    hybrid_store<<<kArcBlocks, 256, 0, st>>>(p);
+    e = cudaGetLastError();
+  }
+  return e;
 }
 
 int hybrid_clusters(int blocks) {

@@ -111,6 +111,13 @@ constexpr int kHybMaxVertices = kResMaxCluster * kHybBlockVertices;
 inline bool hybrid_takes(long long n, long long na, long long longer) {
   return n <= kHybMaxVertices && na < 20 * n && longer <= 2 + n / 256;
 }
+// Above this many vertices and residual arcs a single solve stays with the
+// persistent kernel, whose 152 SMs read the arcs faster.  Persistent and hybrid
+// at 280,000 vertices, BCSR16 and RCSR: random graphs of 5.3M units 1.28, 1.14
+// and 0.75, 1.20 ms, with many terminals of 4.9M 7.9, 7.5 and 8.7, 7.8; below,
+// at 3.6M, 530x530 grids with all pixels terminals 10.7, 5.4 and 11.0, 5.8 ms,
+// but a random graph (13 rounds, 3 relabels) 0.42, 0.66 and 0.54, 0.72.
+constexpr long long kHybMaxUnits = 1 << 22;
 cudaError_t launch_hybrid(const ResParams& p, cudaStream_t st);
 // Clusters of `blocks` (a power of two) of the hybrid solver that run at once.
 int hybrid_clusters(int blocks);
