@@ -22,7 +22,7 @@ INCLUDE = os.path.join(ROOT, "include")
 OUT = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT, "libwbpr.so")
 LIB_CHECKED = os.path.join(OUT, "libwbpr_checked.so")
-CHECKED_SOURCES = ["pr_bcsr.cu", "pr_rcsr.cu"]  # the solver kernels
+CHECKED_SOURCES = ["pr_bcsr.cu", "pr_rcsr.cu", "resident.cu", "hybrid.cu"]  # the solver kernels
 CLI = os.path.join(OUT, "maxflow")
 
 ARCH = ["-gencode=arch=compute_103a,code=sm_103a"]
@@ -99,8 +99,8 @@ def build(force: bool = False, ptxas_verbose: bool = False) -> str:
 
 def build_checked() -> str:
     """libwbpr_checked.so: the solver kernels compiled with bounds-checked
-    arc and vertex accessors (-DWBPR_CHECKED), linked with the other objects
-    of the normal build.  An out-of-range index is counted instead of used,
+    arc and vertex accessors, in global and in shared memory (-DWBPR_CHECKED),
+    linked with the other objects of the normal build.  An out-of-range index is counted instead of used,
     and the solve returns WBPR_ERR_VERIFY.  Built on demand (debugging and
     its GPU test), not by build()."""
     build()

@@ -1859,6 +1859,7 @@ wbpr_status run_resident(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* laun
   g->trace_n = 0;
   *hs = h.st;
   if (flow) *flow = h.flow;
+  if (h.err == (int)WBPR_ERR_VERIFY) g_last_error = "bounds check: out-of-range arc, slot or block indices";
   return (wbpr_status)h.err;
 }
 

@@ -55,7 +55,7 @@ struct HPart {
   int4* rec;
   int rank, cs, shift;     // cs = 1 << shift blocks
   int groups;
-  int n;
+  int n, na;               // vertices and arcs of the instance
   int row0;                // arc number of record 0
   bool rows;               // rows are in shared memory
   int sl, tl;              // s and t among this block's slots, or -1
@@ -69,6 +69,10 @@ struct HPart {
     const int l = s >> 2 & 31, q = (s & 3) * 32 + (l & 7) * 4 + (l >> 3);
     return (q * groups + (s >> 7)) * cs + rank;
   }
+  // a head's memory, its slot there, and an arc, in range
+  __device__ __forceinline__ unsigned mem(int head) const { return Smem::at(a0, within(c, (unsigned)head >> 16, cs)); }
+  __device__ __forceinline__ unsigned at(int head) const { return 4 * within(c, head & 0xffff, 128 * groups); }
+  __device__ __forceinline__ int arc(int a) const { return (int)within(c, a, na); }
   __device__ __forceinline__ int code(int v) const { return (v & (cs - 1)) << 16 | slot(v >> shift); }
 };
 
@@ -107,6 +111,7 @@ __device__ void shape(const ResInstance& in, int4* rec, int cs, HPart& P) {
   P.n = in.n;
   P.rec = rec;
   P.row0 = row_at(in, 0);
+  P.na = row_at(in, in.n) - P.row0;
   P.groups = max(kResThreads >> 5, ((in.n + cs - 1) / cs + 127) >> 7);
 }
 
@@ -128,7 +133,7 @@ __device__ void setup(const ResInstance& in, int4* rec, char* sm, HPart& P) {
   P.sl = P.sv >= 0 && P.sv >> 16 == P.rank ? P.sv & 0xffff : -1;
   P.tl = P.tv >> 16 == P.rank ? P.tv & 0xffff : -1;
   if (threadIdx.x < 8) c->sum[threadIdx.x] = 0;
-  if (threadIdx.x == 0) c->busy[0] = c->busy[1] = c->stop = c->gr = 0;
+  if (threadIdx.x == 0) c->busy[0] = c->busy[1] = c->stop = c->gr = c->viol = 0;
   for (unsigned i = threadIdx.x; i < slots; i += blockDim.x) {
     const int v = P.vertex(i);
     int e = 0, b = 0, d = 0;
@@ -213,9 +218,9 @@ __device__ void write_arcs(const ResInstance& in, const HPart& P, int tid, int n
 // (DIR 0) has residual.
 template <int DIR>
 __device__ __forceinline__ void bfs_arc(const HPart& P, int a, int nl) {
-  const int4 r = record(P.rec, a);
+  const int4 r = record(P.rec, P.arc(a));
   if ((DIR == 0 ? r.y : r.x) <= 0 || r.z == P.sv) return;
-  const unsigned al = Smem::at(P.a0, (unsigned)r.z >> 16) + P.a_lab + 4 * (r.z & 0xffff);
+  const unsigned al = P.mem(r.z) + P.a_lab + P.at(r.z);
   if (Smem::ld(al) > nl) Smem::min(al, nl);
 }
 
@@ -256,12 +261,12 @@ __device__ __forceinline__ void bfs_expand(const ResInstance& in, const HPart& P
   const int2 row = row_of(in, P, u);
   const int nl = (int)lds32(P.a0 + P.a_ex + 4 * u) + 1;
   for (int k = lane; k < row.y; k += 2 * W) {
-    const int4 r = record(P.rec, row.x + k);
+    const int4 r = record(P.rec, P.arc(row.x + k));
     int4 r2 = make_int4(0, 0, P.sv, 0);
-    if (k + W < row.y) r2 = record(P.rec, row.x + k + W);
+    if (k + W < row.y) r2 = record(P.rec, P.arc(row.x + k + W));
     const bool ok = (DIR == 0 ? r.y : r.x) > 0 && r.z != P.sv, ok2 = (DIR == 0 ? r2.y : r2.x) > 0 && r2.z != P.sv;
-    const unsigned al = Smem::at(P.a0, (unsigned)r.z >> 16) + P.a_lab + 4 * (r.z & 0xffff);
-    const unsigned al2 = Smem::at(P.a0, ok2 ? (unsigned)r2.z >> 16 : 0) + P.a_lab + 4 * (r2.z & 0xffff);
+    const int z2 = ok2 ? r2.z : 0;
+    const unsigned al = P.mem(r.z) + P.a_lab + P.at(r.z), al2 = P.mem(z2) + P.a_lab + P.at(z2);
     int l = 0, l2 = 0;
     if (ok) l = Smem::ld(al);
     if (ok2) l2 = Smem::ld(al2);
@@ -338,11 +343,11 @@ __device__ __forceinline__ void discharge(const ResInstance& in, const HPart& P,
     for (int q = 0; q < Q; ++q) {
       const int i = k + q * W + lane;
       r[q] = make_int4(0, 0, 0, 0);
-      if (i < row.y && erem > 0) r[q] = record(P.rec, row.x + i);
+      if (i < row.y && erem > 0) r[q] = record(P.rec, P.arc(row.x + i));
     }
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-      m[q] = Smem::at(P.a0, (unsigned)r[q].z >> 16) + 4 * (r[q].z & 0xffff);
+      m[q] = P.mem(r[q].z) + P.at(r[q].z);
       hv[q] = kBig;
       if (r[q].x > 0) hv[q] = Smem::ld(m[q] + P.a_lab);
     }
@@ -367,8 +372,8 @@ __device__ __forceinline__ void discharge(const ResInstance& in, const HPart& P,
         const int push = (int)min(room[q], left);
         left -= push;
         if (push > 0) {
-          move(P.rec, row.x + k + q * W + lane, push);
-          move(P.rec, r[q].w, -push);
+          move(P.rec, P.arc(row.x + k + q * W + lane), push);
+          move(P.rec, P.arc(r[q].w), -push);
           if (r[q].z == P.tv) sink += push;
           else Smem::add(m[q] + P.a_e, push);
           ++ct.pushes;
@@ -428,7 +433,6 @@ __device__ void solve_hybrid(const ResParams& p, const HPart& P) {
   long long gr_end = 0, gr_len = 0, gr_all = 0;
   const long long clk0 = clock64();
   const unsigned long long t0 = gtime();
-  const int lane = threadIdx.x & 31;
   if (in.mode == kModeBfsOnly) {
     if (in.dir == 0) bfs_hybrid<0>(p, P, seq, ct);
     else bfs_hybrid<1>(p, P, seq, ct);
@@ -437,11 +441,11 @@ __device__ void solve_hybrid(const ResParams& p, const HPart& P) {
       // preflow: every residual arc out of s, by all blocks
       const int b = row_at(in, in.s) - P.row0, e = row_at(in, in.s + 1) - P.row0;
       for (int a = b + P.rank * blockDim.x + threadIdx.x; a < e; a += P.cs * blockDim.x) {
-        const int4 r = record(P.rec, a);
+        const int4 r = record(P.rec, P.arc(a));
         if (r.x <= 0 || r.z == P.sv) continue;
-        move(P.rec, a, r.x);
-        move(P.rec, r.w, -r.x);
-        Smem::add(Smem::at(P.a0, (unsigned)r.z >> 16) + P.a_e + 4 * (r.z & 0xffff), r.x);
+        move(P.rec, P.arc(a), r.x);
+        move(P.rec, P.arc(r.w), -r.x);
+        Smem::add(P.mem(r.z) + P.a_e + P.at(r.z), r.x);
       }
       Smem::sync();
     }
@@ -475,18 +479,11 @@ __device__ void solve_hybrid(const ResParams& p, const HPart& P) {
     }
   }
   if (p.keep) write_back(in, P);
-  if (in.mode != kModeBfsOnly) {
+  if (kChecked || in.mode != kModeBfsOnly) {
     int str = 0;
     for (int i = threadIdx.x; i < 128 * P.groups; i += blockDim.x)
       str += i != P.sl && i != P.tl && (int)lds32(P.a0 + P.a_e + 4 * i) > 0 && (int)lds32(P.a0 + P.a_lab + 4 * i) >= P.n;
-    unsigned long long v[6] = {ct.scanned, ct.bfs, ct.pushes, ct.relabels, ct.visits, (unsigned)str};
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(kFull, v[k], o);
-      if (lane == 0 && v[k]) Smem::add64(Smem::at(P.a0, 0) + (unsigned)offsetof(ResCtl, sum) + 8 * k, v[k]);
-    }
-    Smem::sync();
+    add_up<true>(P.c, P.a0, ct, str);
   }
   report(p.to, P.c, P.rank, in.mode != kModeBfsOnly && P.tl >= 0, P.tl >= 0 ? (int)lds32(P.a0 + P.a_e + 4 * P.tl) : 0, err, rounds, grs, total_levels, gtime() - t0,
          (double)gr_all / (double)(clock64() - clk0));

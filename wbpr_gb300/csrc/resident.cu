@@ -37,7 +37,6 @@
 namespace wbpr_dev {
 namespace {
 
-
 // BFS levels a block runs between two cluster barriers (the search is
 // label-correcting).  GENRMF 16x40: 1 level 4.88, 8 3.76, 32 4.0-5.5 ms;
 // layered 32x256 0.85, 0.53, 0.5-0.8 ms.
@@ -68,6 +67,7 @@ struct Part {
   bool big;                // some row of this block is longer than kBigRow
   int groups;              // of 32 slots, the same in every block
   int nv, na;              // vertices and arcs of this block
+  int arcs;                // there is room for in every block
   int n;                   // of the instance
   int sv, tv;              // s and t as (block << 12 | slot), -1 for none
   int sl, tl;              // s and t among this block's slots, or -1
@@ -75,6 +75,13 @@ struct Part {
     const int q = j / groups;
     return (j - q * groups) * 32 + (q & 3) * 8 + (q >> 2);
   }
+  // the memory of a head's block, the head's {label, excess} and an arc's record there
+  template <bool CL>
+  __device__ __forceinline__ unsigned mem(unsigned head) const {
+    return Sh<CL>::at(a0, within(c, head >> 12, cs));
+  }
+  __device__ __forceinline__ unsigned ve_in(unsigned m, unsigned head) const { return m + a_ve + 8 * within(c, head & 0xfff, 32 * groups); }
+  __device__ __forceinline__ unsigned rec_in(unsigned m, unsigned arc) const { return m + a_rec + 8 * within(c, arc, arcs); }
 };
 
 // First vertex of block k: a 32-way search by one warp over the monotone
@@ -128,7 +135,7 @@ __device__ bool setup(const ResInstance& in, char* sm, Part& P) {
     }
   }
   if (threadIdx.x < 8) c->sum[threadIdx.x] = 0;
-  if (threadIdx.x == 0) c->busy[0] = c->busy[1] = c->stop = c->gr = 0;
+  if (threadIdx.x == 0) c->busy[0] = c->busy[1] = c->stop = c->gr = c->viol = 0;
   __syncthreads();
   int nvmax = 0, namax = 0;
   for (int k = 0; k < P.cs; ++k) {
@@ -136,6 +143,7 @@ __device__ bool setup(const ResInstance& in, char* sm, Part& P) {
     namax = max(namax, c->abase[k + 1] - c->abase[k]);
   }
   P.groups = max((int)blockDim.x >> 5, (nvmax + 31) >> 5);
+  P.arcs = namax;
   const int slots = 32 * P.groups;
   char* q = sm + ((sizeof(ResCtl) + 15) & ~15u);
   P.rec = (int2*)q;
@@ -213,8 +221,9 @@ __device__ void load(const ResInstance& in, Part& P) {
 #pragma unroll 4
     for (int a = threadIdx.x; a < P.na; a += blockDim.x) {
       const int2 r = __ldcg(in.arc + a0 + a), x = __ldg(in.arx + a0 + a);
-      const int d = r.x - in.vbase, o = owner_of(c, P.cs, d);
-      P.rec[a] = make_int2(fresh ? x.y : r.y, (int)((unsigned)(o << 12 | P.slot(d - c->bnd[o])) | (unsigned)(x.x - c->abase[o]) << 16));
+      const int d = (int)within(P.c, r.x - in.vbase, P.n), o = owner_of(c, P.cs, d);
+      const unsigned tw = within(P.c, x.x - c->abase[o], P.arcs);
+      P.rec[a] = make_int2(fresh ? x.y : r.y, (int)((unsigned)(o << 12 | P.slot(d - c->bnd[o])) | tw << 16));
     }
     Sh<CL>::sync();
     return;
@@ -223,17 +232,19 @@ __device__ void load(const ResInstance& in, Part& P) {
   for_rows(P, [&](int j, int k) {
     const int v = v0 + j, fb = __ldg(in.frow + v), nf = __ldg(in.frow + v + 1) - fb;
     const int here = (int)(P.row[P.slot(j)] & 0xffff) + k;
-    int2* q = P.rec + here;
+    int2* q = P.rec + within(P.c, here, P.arcs);
     if (k < nf) {
-      const int2 r = __ldcg(in.farc + fb + k);
+      int2 r = __ldcg(in.farc + fb + k);
+      r.x = (int)within(P.c, r.x, P.n);
       const int o = owner_of(c, P.cs, r.x);
       q->x = fresh ? __ldg(in.fcap + fb + k) : r.y;
       *(unsigned short*)&q->y = (unsigned short)(o << 12 | P.slot(r.x - c->bnd[o]));  // its twin is written below
     } else {
-      const int2 r = __ldg(in.rarc + __ldg(in.rrow + v) + k - nf);  // {tail, forward arc}
+      int2 r = __ldg(in.rarc + __ldg(in.rrow + v) + k - nf);  // {tail, forward arc}
+      r.x = (int)within(P.c, r.x, P.n);
       const int o = owner_of(c, P.cs, r.x);
-      const int tw = r.y + __ldg(in.rrow + r.x) - c->abase[o];
-      *q = make_int2(fresh ? 0 : __ldcg(in.fcb + r.y), (int)((unsigned)(o << 12 | P.slot(r.x - c->bnd[o])) | (unsigned)tw << 16));
+      const unsigned tw = within(P.c, r.y + __ldg(in.rrow + r.x) - c->abase[o], P.arcs);
+      *q = make_int2(fresh ? 0 : __ldcg(in.fcb + r.y), (int)((unsigned)(o << 12 | P.slot(r.x - c->bnd[o])) | tw << 16));
       Sh<CL>::st16(Sh<CL>::at(P.a0, o) + P.a_rec + 8 * tw + 6, (unsigned)here);
     }
   });
@@ -268,14 +279,14 @@ template <int W, bool CL, int DIR>
 __device__ __forceinline__ void bfs_expand(const Part& P, int u, int l, Count& ct) {
   const unsigned lane = threadIdx.x & (W - 1);
   const unsigned row = u >= 0 ? lds32(P.a_row + 4 * u) : 0;
-  const unsigned deg = row >> 16, rec = P.a0 + P.a_rec + 8 * (row & 0xffff);
+  const unsigned deg = row >> 16, first = row & 0xffff;
   const int nl = l + 1;
   for (unsigned k = lane; k < deg; k += W) {
-    const int2 r = lds64(rec + 8 * k);
+    const int2 r = lds64(P.rec_in(P.a0, first + k));
     if (DIR == 1 && r.x <= 0) continue;
-    const unsigned d = r.y & 0xffff, m = Sh<CL>::at(P.a0, d >> 12), al = m + P.a_ve + 8 * (d & 0xfff);
+    const unsigned d = r.y & 0xffff, m = P.mem<CL>(d), al = P.ve_in(m, d);
     const int lv = Sh<CL>::ld(al);
-    const int cf = DIR == 0 ? Sh<CL>::ld(m + P.a_rec + 8 * ((unsigned)r.y >> 16)) : 1;
+    const int cf = DIR == 0 ? Sh<CL>::ld(P.rec_in(m, (unsigned)r.y >> 16)) : 1;
     if (lv > nl && cf > 0 && (int)d != P.sv) Sh<CL>::min(al, nl);
   }
   if (lane == 0) ct.bfs += deg;
@@ -351,7 +362,7 @@ __device__ __forceinline__ void discharge(const Part& P, int u, Count& ct) {
     le = lds64(P.a0 + P.a_ve + 8 * u);  // one read by the tile's lanes together
     row = lds32(P.a_row + 4 * u);
   }
-  const unsigned deg = row >> 16, rec = P.a0 + P.a_rec + 8 * (row & 0xffff);
+  const unsigned deg = row >> 16, first = row & 0xffff;
   const int hu = le.x;
   unsigned erem = (unsigned)le.y, k = 0;
   int mn = kBig;
@@ -364,13 +375,13 @@ __device__ __forceinline__ void discharge(const Part& P, int u, Count& ct) {
     for (int q = 0; q < Q; ++q) {
       const unsigned i = k + q * W + lane;
       r[q] = make_int2(0, 0);
-      if (i < deg && erem > 0) r[q] = lds64(rec + 8 * i);
+      if (i < deg && erem > 0) r[q] = lds64(P.rec_in(P.a0, first + i));
     }
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-      m[q] = Sh<CL>::at(P.a0, (r[q].y & 0xf000) >> 12);
+      m[q] = P.mem<CL>(r[q].y & 0xffff);
       hv[q] = kBig;
-      if (r[q].x > 0) hv[q] = Sh<CL>::ld(m[q] + P.a_ve + 8 * (r[q].y & 0xfff));
+      if (r[q].x > 0) hv[q] = Sh<CL>::ld(P.ve_in(m[q], r[q].y & 0xffff));
     }
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
@@ -394,9 +405,9 @@ __device__ __forceinline__ void discharge(const Part& P, int u, Count& ct) {
         const int push = (int)min(room[q], left);
         left -= push;
         if (push > 0) {
-          Sh<false>::add(rec + 8 * (k + q * W + lane), -push);
-          Sh<CL>::add(m[q] + P.a_rec + 8 * ((unsigned)r[q].y >> 16), push);
-          Sh<CL>::add(m[q] + P.a_ve + 8 * (r[q].y & 0xfff) + 4, push);
+          Sh<false>::add(P.rec_in(P.a0, first + k + q * W + lane), -push);
+          Sh<CL>::add(P.rec_in(m[q], (unsigned)r[q].y >> 16), push);
+          Sh<CL>::add(P.ve_in(m[q], r[q].y & 0xffff) + 4, push);
           ++ct.pushes;
         }
         if (r[q].x > push) mn = min(mn, hv[q]);
@@ -458,7 +469,6 @@ __device__ void solve_resident(const ResParams& p, Part& P) {
   long long gr_end = 0, gr_len = 0, gr_all = 0;
   const long long clk0 = clock64();
   const unsigned long long t0 = gtime();
-  const int lane = threadIdx.x & 31;
   if (in.mode == kModeBfsOnly) {
     if (in.dir == 0) bfs_resident<W, CL, 0>(p, P, seq, ct);
     else bfs_resident<W, CL, 1>(p, P, seq, ct);
@@ -469,11 +479,11 @@ __device__ void solve_resident(const ResParams& p, Part& P) {
       for (int k = threadIdx.x; k < (int)(row >> 16); k += blockDim.x) {
         const int a = (row & 0xffff) + k;
         const int2 r = P.rec[a];
-        const unsigned d = r.y & 0xffff, m = Sh<CL>::at(P.a0, d >> 12);
+        const unsigned d = r.y & 0xffff, m = P.mem<CL>(d);
         if (r.x <= 0 || (int)d == P.sv) continue;
         P.rec[a].x = 0;
-        Sh<CL>::add(m + P.a_rec + 8 * ((unsigned)r.y >> 16), r.x);
-        Sh<CL>::add(m + P.a_ve + 8 * (d & 0xfff) + 4, r.x);
+        Sh<CL>::add(P.rec_in(m, (unsigned)r.y >> 16), r.x);
+        Sh<CL>::add(P.ve_in(m, d) + 4, r.x);
       }
     }
     Sh<CL>::sync();
@@ -513,19 +523,11 @@ __device__ void solve_resident(const ResParams& p, Part& P) {
     }
   }
   if (p.keep) write_back(in, P);
-  // counters: warps into the block's words, blocks into the first block's
-  if (in.mode != kModeBfsOnly) {
+  if (kChecked || in.mode != kModeBfsOnly) {
     int str = 0;
     for (int i = threadIdx.x; i < 32 * P.groups; i += blockDim.x)
       str += i != P.sl && i != P.tl && P.ve[i].y > 0 && P.ve[i].x >= P.n;
-    unsigned long long v[6] = {ct.scanned, ct.bfs, ct.pushes, ct.relabels, ct.visits, (unsigned)str};
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(kFull, v[k], o);
-      if (lane == 0 && v[k]) Sh<CL>::add64(Sh<CL>::at(P.a0, 0) + (unsigned)offsetof(ResCtl, sum) + 8 * k, v[k]);
-    }
-    Sh<CL>::sync();
+    add_up<CL>(P.c, P.a0, ct, str);
   }
   report(p.to, P.c, P.rank, in.mode != kModeBfsOnly && P.tl >= 0, P.tl >= 0 ? P.ve[P.tl].y : 0, err, rounds, grs, total_levels, gtime() - t0,
          (double)gr_all / (double)(clock64() - clk0));
@@ -571,7 +573,7 @@ int resident_cluster(long long n, long long na) {
 
 cudaError_t launch_resident(const ResParams& p0, int tile, int cluster, cudaStream_t st) {
   ResParams p = p0;
-    p.run.bsub = cluster == 1 ? 1 : kResBfsLevels;
+  p.run.bsub = cluster == 1 ? 1 : kResBfsLevels;
   p.run.grp = cluster == 1 ? kResGrShareBlock : kResGrShare;
   if (cluster == 1) return tile < 32 ? launch_cluster<pr_resident<8, false>>(p, 1, st) : launch_cluster<pr_resident<32, false>>(p, 1, st);
   return tile < 32 ? launch_cluster<pr_resident<8, true>>(p, cluster, st) : launch_cluster<pr_resident<32, true>>(p, cluster, st);

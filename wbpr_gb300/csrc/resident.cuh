@@ -22,8 +22,22 @@ struct ResCtl {
   int stop;                       // number of the barrier after which every block stops: budget exhausted
   int gr;                         // number of the barrier after which every block relabels globally
   int item;                       // the claimed instance of a batch
+  int viol;                       // checked build: indices of this block out of range
   unsigned long long sum[8];      // counters
 };
+
+// The checked build (compiled with -DWBPR_CHECKED): an index outside [0, lim) is
+// counted, replaced by 0, and the solve returns WBPR_ERR_VERIFY.
+#ifdef WBPR_CHECKED
+constexpr bool kChecked = true;
+#else
+constexpr bool kChecked = false;
+#endif
+__device__ __forceinline__ unsigned within(ResCtl* c, unsigned i, unsigned lim) {
+  if (!kChecked || i < lim) return i;
+  atomicAdd(&c->viol, 1);
+  return 0;
+}
 
 __device__ __forceinline__ unsigned sm_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ unsigned cl_rank() {
@@ -123,12 +137,29 @@ __device__ __forceinline__ int row_at(const ResInstance& in, int v) {
   return in.row ? __ldg(in.row + in.vbase + v) : __ldg(in.frow + v) + __ldg(in.rrow + v);
 }
 
+// The counters of one solve: warps into the block's words, blocks into the
+// first block's.  A barrier.
+template <bool CL>
+__device__ __forceinline__ void add_up(ResCtl* c, unsigned a0, const Count& ct, int stranded) {
+  if (kChecked) __syncthreads();  // every index has been checked
+  unsigned long long v[7] = {ct.scanned, ct.bfs, ct.pushes, ct.relabels, ct.visits, (unsigned)stranded,
+                             kChecked && threadIdx.x == 0 ? (unsigned)c->viol : 0};
+#pragma unroll
+  for (int k = 0; k < (kChecked ? 7 : 6); ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(kFull, v[k], o);
+    if ((threadIdx.x & 31) == 0 && v[k]) Sh<CL>::add64(Sh<CL>::at(a0, 0) + (unsigned)offsetof(ResCtl, sum) + 8 * k, v[k]);
+  }
+  Sh<CL>::sync();
+}
+
 // Writes the results of one solve (called by every thread of the cluster
 // behind the barrier after which c->sum is complete); `mine`: this block owns
 // t, whose excess is `flow`.
 __device__ __forceinline__ void report(const ResReport& to, const ResCtl* c, int rank, bool mine, int flow, int err, int rounds, int grs,
                                        int levels, unsigned long long ns, double gr_share) {
   if (threadIdx.x != 0) return;
+  if (kChecked && rank == 0 && c->sum[6]) err = (int)WBPR_ERR_VERIFY;
   if (mine) {
     if (to.out) to.out->flow = flow;
     else *to.flow = err ? -1 : flow;
