@@ -72,3 +72,31 @@ def test_checked_shared_memory_solvers_stay_in_bounds():
         want.append(oracle.dinic(g.n, g.off, g.dst, g.cap, g.s, g.t))
     assert rows == [[v] * 12 for v in want]
     assert flows == want
+
+
+def _alone(body):
+    """Runs a program on the checked build in a process of its own."""
+    head = "import sys\nsys.path[:0] = [%r, %r]\nimport numpy as np\nimport oracle\nimport wbpr_gb300 as W\n"
+    r = subprocess.run([sys.executable, "-c", head % (ROOT, os.path.join(ROOT, "tests")) + body], capture_output=True,
+                       text=True, env=dict(os.environ, WBPR_CHECKED="1"), timeout=1200)
+    assert r.returncode == 0, r.stdout[-1000:] + r.stderr[-3000:]
+
+
+@pytest.mark.gpu
+def test_the_blocks_of_a_cluster_decide_alike():
+    """When to relabel globally and when to give up hangs on a clock, which the
+    lanes of a warp read at different times in this build: the blocks must all
+    get one lane's answer.  Many relabels, and budgets that run out at any point."""
+    _alone(r"""
+for g in (W.gen_genrmf(8, 16, 1, 10000, 4), W.gen_genrmf(12, 20, 1, 10000, 3), W.gen_layered(31, 641, 3, 6, 1, 1000, 8)):
+    want = oracle.dinic(g.n, g.off, g.dst, g.cap, g.s, g.t)
+    for layout in ("bcsr", "rcsr"):
+        with W.DeviceGraph(g, layout) as d:
+            for kw in [dict(max_ms=x) for x in (1e-3, 0.05, 0.2, 0.5)] + [dict(max_rounds=x) for x in (1, 5, 12)]:
+                try:
+                    assert d.solve("vc", **kw).flow == want
+                except W.WbprError as e:
+                    assert e.status == 3, e
+            r = d.solve("vc")
+            assert r.flow == want and r.global_relabels > 1 and d.verify()["ok"]
+""")

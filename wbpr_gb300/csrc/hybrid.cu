@@ -430,9 +430,7 @@ __device__ void solve_hybrid(const ResParams& p, const HPart& P) {
   const ResInstance& in = p.in;
   Count ct;
   int seq = 0, grs = 0, rounds = 0, since = 0, err = 0, total_levels = 0;
-  long long gr_end = 0, gr_len = 0, gr_all = 0;
-  const long long clk0 = clock64();
-  const unsigned long long t0 = gtime();
+  solve_begins(P.c);
   if (in.mode == kModeBfsOnly) {
     if (in.dir == 0) bfs_hybrid<0>(p, P, seq, ct);
     else bfs_hybrid<1>(p, P, seq, ct);
@@ -452,22 +450,14 @@ __device__ void solve_hybrid(const ResParams& p, const HPart& P) {
     bool need_gr = true;
     for (;;) {
       if (need_gr) {
-        const long long c0 = clock64();
+        relabel_begins(P.c);
         total_levels += bfs_hybrid<0>(p, P, seq, ct);
-        gr_end = clock64();
-        gr_len = gr_end - c0;
-        gr_all += gr_len;
+        relabel_ends(P.c);
         ++grs;
         since = 0;
       }
       const bool did = push_step(in, P, ct);
-      if (P.rank == 0 && threadIdx.x < P.cs) {
-        const unsigned to = Smem::at(P.a0, threadIdx.x);
-        const bool out_of_time = (unsigned long long)(clock64() - clk0) >= p.run.budget_ns >> 1 && time_past(t0, p.run.budget_ns);
-        if ((p.run.max_rounds > 0 && rounds >= p.run.max_rounds) || out_of_time)
-          Smem::st(to + (unsigned)offsetof(ResCtl, stop), seq + 1);
-        if (since >= 8 && (clock64() - gr_end) * 16 >= gr_len * p.run.grp) Smem::st(to + (unsigned)offsetof(ResCtl, gr), seq + 1);
-      }
+      decide<true>(P.c, P.a0, P.rank, P.cs, p.run, rounds, since, seq);
       if (!any_work<true>(P.c, P.a0, P.cs, did, seq)) break;
       if (*(volatile int*)&P.c->stop == seq) {
         err = (int)WBPR_ERR_NO_CONVERGENCE;
@@ -485,8 +475,7 @@ __device__ void solve_hybrid(const ResParams& p, const HPart& P) {
       str += i != P.sl && i != P.tl && (int)lds32(P.a0 + P.a_e + 4 * i) > 0 && (int)lds32(P.a0 + P.a_lab + 4 * i) >= P.n;
     add_up<true>(P.c, P.a0, ct, str);
   }
-  report(p.to, P.c, P.rank, in.mode != kModeBfsOnly && P.tl >= 0, P.tl >= 0 ? (int)lds32(P.a0 + P.a_e + 4 * P.tl) : 0, err, rounds, grs, total_levels, gtime() - t0,
-         (double)gr_all / (double)(clock64() - clk0));
+  report(p.to, P.c, P.rank, in.mode != kModeBfsOnly && P.tl >= 0, P.tl >= 0 ? (int)lds32(P.a0 + P.a_e + 4 * P.tl) : 0, err, rounds, grs, total_levels);
 }
 
 extern __shared__ __align__(16) char hyb_smem[];

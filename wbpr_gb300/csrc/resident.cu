@@ -466,9 +466,7 @@ __device__ void solve_resident(const ResParams& p, Part& P) {
   const ResInstance& in = p.in;
   Count ct;
   int seq = 0, grs = 0, rounds = 0, since = 0, err = 0, total_levels = 0;
-  long long gr_end = 0, gr_len = 0, gr_all = 0;
-  const long long clk0 = clock64();
-  const unsigned long long t0 = gtime();
+  solve_begins(P.c);
   if (in.mode == kModeBfsOnly) {
     if (in.dir == 0) bfs_resident<W, CL, 0>(p, P, seq, ct);
     else bfs_resident<W, CL, 1>(p, P, seq, ct);
@@ -490,26 +488,14 @@ __device__ void solve_resident(const ResParams& p, Part& P) {
     bool need_gr = true;
     for (;;) {
       if (need_gr) {
-        const long long c0 = clock64();
+        relabel_begins(P.c);
         total_levels += bfs_resident<W, CL, 0>(p, P, seq, ct);
-        gr_end = clock64();
-        gr_len = gr_end - c0;
-        gr_all += gr_len;
+        relabel_ends(P.c);
         ++grs;
         since = 0;
       }
       const bool did = push_step<W, CL>(P, ct);
-      // the first block decides, and posts the number of the barrier below
-      // (not a flag: a slow block may read the word only after a fast one has
-      // reached the next barrier)
-      if (P.rank == 0 && threadIdx.x < P.cs) {
-        const unsigned to = Sh<CL>::at(P.a0, threadIdx.x);
-        // the cycle counter first (cheaper to read; an SM does over half a cycle per ns)
-        const bool out_of_time = (unsigned long long)(clock64() - clk0) >= p.run.budget_ns >> 1 && time_past(t0, p.run.budget_ns);
-        if ((p.run.max_rounds > 0 && rounds >= p.run.max_rounds) || out_of_time)
-          Sh<CL>::st(to + (unsigned)offsetof(ResCtl, stop), seq + 1);
-        if (since >= 8 && (clock64() - gr_end) * 16 >= gr_len * p.run.grp) Sh<CL>::st(to + (unsigned)offsetof(ResCtl, gr), seq + 1);
-      }
+      decide<CL>(P.c, P.a0, P.rank, P.cs, p.run, rounds, since, seq);
       // the labels are valid after every step, so no active vertex means a
       // maximum preflow
       if (!any_work<CL>(P.c, P.a0, P.cs, did, seq)) break;
@@ -529,8 +515,7 @@ __device__ void solve_resident(const ResParams& p, Part& P) {
       str += i != P.sl && i != P.tl && P.ve[i].y > 0 && P.ve[i].x >= P.n;
     add_up<CL>(P.c, P.a0, ct, str);
   }
-  report(p.to, P.c, P.rank, in.mode != kModeBfsOnly && P.tl >= 0, P.tl >= 0 ? P.ve[P.tl].y : 0, err, rounds, grs, total_levels, gtime() - t0,
-         (double)gr_all / (double)(clock64() - clk0));
+  report(p.to, P.c, P.rank, in.mode != kModeBfsOnly && P.tl >= 0, P.tl >= 0 ? P.ve[P.tl].y : 0, err, rounds, grs, total_levels);
 }
 
 extern __shared__ __align__(16) char res_smem[];

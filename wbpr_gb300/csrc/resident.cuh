@@ -24,6 +24,10 @@ struct ResCtl {
   int item;                       // the claimed instance of a batch
   int viol;                       // checked build: indices of this block out of range
   unsigned long long sum[8];      // counters
+  // times of the solve, kept by the block's first thread: cycle counter and ns
+  // at its start, end and length of the last global relabel, length of all
+  long long clk0, gr_end, gr_len, gr_all;
+  unsigned long long t0;
 };
 
 // The checked build (compiled with -DWBPR_CHECKED): an index outside [0, lim) is
@@ -128,6 +132,12 @@ __device__ __forceinline__ bool any_work(ResCtl* c, unsigned a0, int cs, bool di
   return *(volatile int*)&c->busy[seq & 1] == seq;
 }
 
+// Nothing keeps the lanes of a warp together where they need not be: the
+// checked build calls this to have them come one after the other.
+__device__ __forceinline__ void lanes_apart() {
+  if (kChecked) __nanosleep(64 * (threadIdx.x & 31));
+}
+
 struct Count {  // of one thread
   unsigned scanned = 0, bfs = 0, pushes = 0, relabels = 0, visits = 0;
 };
@@ -153,12 +163,56 @@ __device__ __forceinline__ void add_up(ResCtl* c, unsigned a0, const Count& ct, 
   Sh<CL>::sync();
 }
 
+// The times of a solve, of a global relabel and between the two.
+__device__ __forceinline__ void solve_begins(ResCtl* c) {
+  if (threadIdx.x != 0) return;
+  c->clk0 = clock64();
+  c->t0 = gtime();
+  c->gr_all = 0;
+}
+__device__ __forceinline__ void relabel_begins(ResCtl* c) {
+  if (threadIdx.x == 0) c->gr_len = -clock64();
+}
+__device__ __forceinline__ void relabel_ends(ResCtl* c) {
+  if (threadIdx.x != 0) return;
+  c->gr_end = clock64();
+  c->gr_len += c->gr_end;
+  c->gr_all += c->gr_len;
+}
+
+// Whether the cluster stops (a budget is exhausted) or relabels globally after
+// its next barrier, number seq + 1: one lane of the first block decides, and its
+// warp posts the number to every block.  (Not a flag: a slow block may read the
+// word only after a fast one has reached the barrier after it.  Not every lane
+// for its own block: they could read the clock at different times, and blocks
+// that decided differently would wait for each other forever.)
+template <bool CL>
+__device__ __forceinline__ void decide(ResCtl* c, unsigned a0, int rank, int cs, const ResRun& run, int rounds, int since, int seq) {
+  if (rank != 0 || threadIdx.x >= 32) return;
+  bool stop = false, gr = false;
+  lanes_apart();
+  if (threadIdx.x == 0) {
+    // the cycle counter first (cheaper to read; an SM does over half a cycle per ns)
+    const long long now = clock64();
+    stop = (run.max_rounds > 0 && rounds >= run.max_rounds) ||
+           ((unsigned long long)(now - c->clk0) >= run.budget_ns >> 1 && time_past(c->t0, run.budget_ns));
+    gr = since >= 8 && (now - c->gr_end) * 16 >= c->gr_len * run.grp;
+  }
+  stop = __shfl_sync(kFull, stop, 0);
+  gr = __shfl_sync(kFull, gr, 0);
+  if ((int)threadIdx.x >= cs) return;
+  const unsigned to = Sh<CL>::at(a0, threadIdx.x);
+  if (stop) Sh<CL>::st(to + (unsigned)offsetof(ResCtl, stop), seq + 1);
+  if (gr) Sh<CL>::st(to + (unsigned)offsetof(ResCtl, gr), seq + 1);
+}
+
 // Writes the results of one solve (called by every thread of the cluster
 // behind the barrier after which c->sum is complete); `mine`: this block owns
 // t, whose excess is `flow`.
 __device__ __forceinline__ void report(const ResReport& to, const ResCtl* c, int rank, bool mine, int flow, int err, int rounds, int grs,
-                                       int levels, unsigned long long ns, double gr_share) {
+                                       int levels) {
   if (threadIdx.x != 0) return;
+  const unsigned long long ns = gtime() - c->t0;
   if (kChecked && rank == 0 && c->sum[6]) err = (int)WBPR_ERR_VERIFY;
   if (mine) {
     if (to.out) to.out->flow = flow;
@@ -180,7 +234,7 @@ __device__ __forceinline__ void report(const ResReport& to, const ResCtl* c, int
   s.rounds = rounds;
   s.grs = grs;
   s.bfs_levels = levels;
-  s.gr_ns = (unsigned long long)((double)ns * gr_share);
+  s.gr_ns = (unsigned long long)((double)ns * ((double)c->gr_all / (double)(clock64() - c->clk0)));
   s.push_ns = s.round_ns = ns - s.gr_ns;
   to.out->st = s;
   to.out->err = err;
