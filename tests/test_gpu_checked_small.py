@@ -100,3 +100,29 @@ for g in (W.gen_genrmf(8, 16, 1, 10000, 4), W.gen_genrmf(12, 20, 1, 10000, 3), W
             r = d.solve("vc")
             assert r.flow == want and r.global_relabels > 1 and d.verify()["ok"]
 """)
+
+
+@pytest.mark.gpu
+def test_a_tile_works_on_one_value_of_the_excess():
+    """Vertices that many others push to while their own tile pushes on: with the
+    lanes of a tile apart, every unit must still be counted once."""
+    _alone(r"""
+rng = np.random.default_rng(5)
+n, hubs = 3000, 24
+tail, head = rng.integers(0, n, 30000), rng.integers(0, n, 30000)
+tail[::3], head[1::3] = rng.integers(1, hubs, 10000), rng.integers(1, hubs, 10000)
+for g in (W.Graph.from_arcs(n, tail, head, rng.integers(1, 1000, 30000), 0, n - 1), W.gen_rmat(10, 16, seed=4),
+          W.gen_rmat(13, 12, seed=4), W.gen_genrmf(9, 9, 1, 100, 2), W.gen_grid(150, 170, 3)):
+    want = oracle.dinic(g.n, g.off, g.dst, g.cap, g.s, g.t)
+    tails = np.repeat(np.arange(g.n), np.diff(g.off))
+    for layout in ("bcsr", "rcsr"):
+        with W.DeviceGraph(g, layout) as d:
+            for _ in range(3):
+                assert d.solve("vc").flow == want and d.verify()["ok"]
+                _, e, f = d.read_state()
+                net = np.zeros(g.n, np.int64)
+                np.add.at(net, g.dst, f)
+                np.add.at(net, tails, -f.astype(np.int64))
+                net[g.s] = e[g.s]
+                assert (net == e).all()
+""")

@@ -345,7 +345,10 @@ __device__ int bfs_resident(const ResParams& p, Part& P, int& seq, Count& ct) {
 }
 
 // Push and relabel the active vertices in slots u (one per W-lane tile, -1
-// for none; whole warps call it).  A vertex's own label is the one it had when
+// for none; whole warps call it) that hold E.  Other warps and blocks add to a
+// vertex's excess meanwhile, so E is what one lane read for all of them: lanes
+// that read it each for themselves could see different values, and what they
+// push would not be what the vertex loses.  A vertex's own label is the one it had when
 // the step began; a head's label may be read before or after that head's
 // relabel of the step.  An arc is admissible when the head's label is lower.
 // Of the two ends of an arc at most one can push along it in a step, because
@@ -354,17 +357,17 @@ __device__ int bfs_resident(const ResParams& p, Part& P, int& seq, Count& ct) {
 // step into u that this scan has not seen: they come from labels at most one
 // above u's.
 template <int W, bool CL>
-__device__ __forceinline__ void discharge(const Part& P, int u, Count& ct) {
+__device__ __forceinline__ void discharge(const Part& P, int u, int E, Count& ct) {
   const unsigned lane = threadIdx.x & (W - 1);
-  int2 le = make_int2(0, 0);
+  lanes_apart();
   unsigned row = 0;
+  int hu = 0;  // no other warp writes it
   if (u >= 0) {
-    le = lds64(P.a0 + P.a_ve + 8 * u);  // one read by the tile's lanes together
+    hu = (int)lds32(P.a0 + P.a_ve + 8 * u);
     row = lds32(P.a_row + 4 * u);
   }
   const unsigned deg = row >> 16, first = row & 0xffff;
-  const int hu = le.x;
-  unsigned erem = (unsigned)le.y, k = 0;
+  unsigned erem = (unsigned)E, k = 0;
   int mn = kBig;
   constexpr int Q = 2;
   do {
@@ -430,7 +433,7 @@ __device__ __forceinline__ void discharge(const Part& P, int u, Count& ct) {
   if (lane == 0 && u >= 0) {
     ct.scanned += min(k, deg);
     ++ct.visits;
-    if (le.y > (int)erem) Sh<false>::add(P.a0 + P.a_ve + 8 * u + 4, (int)erem - le.y);
+    if (E > (int)erem) Sh<false>::add(P.a0 + P.a_ve + 8 * u + 4, (int)erem - E);
   }
 }
 
@@ -449,12 +452,16 @@ __device__ __forceinline__ bool push_step(const Part& P, Count& ct) {
     if (W < 32 && P.big) {
       unsigned big = __ballot_sync(kFull, act && P.row[i] >> 16 > kBigRow);
       mask &= ~big;
-      for (; big; big &= big - 1) discharge<32, CL>(P, g * 32 + __ffs(big) - 1, ct);
+      for (; big; big &= big - 1) {
+        const int t = __ffs(big) - 1;
+        discharge<32, CL>(P, g * 32 + t, __shfl_sync(kFull, le.y, t), ct);
+      }
     }
     // a tile takes the active ones among its own W slots
     unsigned mine = W == 32 ? mask : mask >> (lane & ~(W - 1)) & ((1u << (W & 31)) - 1u);
     while (__any_sync(kFull, mine)) {
-      discharge<W, CL>(P, mine ? g * 32 + (lane & ~(W - 1)) + __ffs(mine) - 1 : -1, ct);
+      const int t = __ffs(mine) - 1, E = __shfl_sync(kFull, le.y, t & (W - 1), W);
+      discharge<W, CL>(P, mine ? g * 32 + (lane & ~(W - 1)) + t : -1, mine ? E : 0, ct);
       mine &= mine - 1;
     }
   }
