@@ -596,12 +596,15 @@ wbpr_status capture(wbpr_batch* b, int tile, int block, double alpha, int grr, l
   BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   cudaError_t e = cudaMemsetAsync(b->next, 0, kLists * sizeof(int), b->stream);
   cudaEventRecord(b->fork, b->stream);
+  // `stream` waits for the branches only behind the launch of its own: that one
+  // would otherwise start when all of them have ended
+  bool joined[wbpr_batch::kSides] = {};
   auto branch = [&](int k, auto launch) {
     cudaStreamWaitEvent(b->side[k], b->fork, 0);
     const cudaError_t x = launch(b->side[k]);
     if (e == cudaSuccess) e = x;
     cudaEventRecord(b->join[k], b->side[k]);
-    cudaStreamWaitEvent(b->stream, b->join[k], 0);
+    joined[k] = true;
   };
   for (int k = 0; k < kHybClasses; ++k) {
     if (!hyb_clusters[k]) continue;
@@ -626,6 +629,8 @@ wbpr_status capture(wbpr_batch* b, int tile, int block, double alpha, int grr, l
     const cudaError_t x = cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, b->stream);
     if (e == cudaSuccess) e = x;
   }
+  for (int k = 0; k < wbpr_batch::kSides; ++k)
+    if (joined[k]) cudaStreamWaitEvent(b->stream, b->join[k], 0);
   const cudaError_t end = cudaStreamEndCapture(b->stream, &graph);
   if (e == cudaSuccess) e = end;
   if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec, graph, 0);
