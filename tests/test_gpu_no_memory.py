@@ -1,0 +1,48 @@
+"""Calls that ask for device memory beyond what their handle holds, when there
+is none: what another path can do without it is done there.  The checked build
+refuses pool requests from a given size on; nothing is really exhausted.  Run in
+a process of its own, which loads that build."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+pytestmark = pytest.mark.gpu
+
+HEAD = r"""
+import ctypes as C, sys
+sys.path[:0] = [%r, %r]
+import numpy as np
+import oracle
+import wbpr_gb300 as W
+
+def refuse(from_bytes):
+    f = W.lib().wbpr_checked_refuse_from
+    f.argtypes, f.restype = [C.c_int64], None
+    f(from_bytes)
+
+def exact(g):
+    return oracle.dinic(g.n, g.off, g.dst, g.cap, g.s, g.t)
+""" % (ROOT, os.path.join(ROOT, "tests"))
+
+
+def run(body):
+    r = subprocess.run([sys.executable, "-c", HEAD + body], capture_output=True, text=True, timeout=600,
+                       env=dict(os.environ, WBPR_CHECKED="1"))
+    assert r.returncode == 0, r.stdout[-1000:] + r.stderr[-3000:]
+
+
+def test_a_solve_without_room_for_arc_records():
+    run(r"""
+for layout in ("bcsr", "rcsr"):
+    g = W.gen_layered(31, 641, 3, 6, 1, 1000, 8)  # the hybrid solver's: 16 bytes a residual arc
+    with W.DeviceGraph(g, layout) as d:
+        refuse(1 << 20)
+        assert d.solve("vc").flow == exact(g) and d.verify()["ok"]
+        held = d.device_bytes
+        refuse(0)
+        assert d.solve("vc").flow == exact(g) and d.verify()["ok"] and d.device_bytes == held
+""")

@@ -22,7 +22,8 @@ INCLUDE = os.path.join(ROOT, "include")
 OUT = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT, "libwbpr.so")
 LIB_CHECKED = os.path.join(OUT, "libwbpr_checked.so")
-CHECKED_SOURCES = ["pr_bcsr.cu", "pr_rcsr.cu", "resident.cu", "hybrid.cu"]  # the solver kernels
+# the solver kernels, and the allocator (whose requests the checked build can refuse)
+CHECKED_SOURCES = ["pr_bcsr.cu", "pr_rcsr.cu", "resident.cu", "hybrid.cu", "graph_dev.cu"]
 CLI = os.path.join(OUT, "maxflow")
 
 ARCH = ["-gencode=arch=compute_103a,code=sm_103a"]

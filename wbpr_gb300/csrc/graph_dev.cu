@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <limits>
@@ -59,7 +60,15 @@ cudaMemPool_t device_pool(int device) {
   return g_pools[device];
 }
 
+#ifdef WBPR_CHECKED
+std::atomic<long long> g_refuse_from{0};  // pool requests of at least this many bytes fail (0: none)
+#endif
+
 cudaError_t pool_alloc_on(void** p, size_t bytes, cudaStream_t stream) {
+#ifdef WBPR_CHECKED
+  const long long refuse = g_refuse_from.load();
+  if (refuse > 0 && bytes >= (size_t)refuse) return cudaErrorMemoryAllocation;
+#endif
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -1799,7 +1808,8 @@ bool use_resident(const wbpr_graph* g, const RunCfg& rc) {
 
 // One launch of the resident or the hybrid solver.  *fits is cleared when
 // neither can take the graph after all (a row too long for a block's share, a
-// device without such clusters); nothing has changed then.
+// device without such clusters, no memory for the records); nothing has
+// changed then.
 wbpr_status run_resident(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch_ms, int* flow, bool* fits) {
   *fits = true;
   ResInstance in{};
@@ -1828,9 +1838,9 @@ wbpr_status run_resident(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* laun
       *fits = false;
       return WBPR_OK;
     }
-    if (g->res_cluster == 0 && !g->hyb_rec) {
-      wbpr_status st = dalloc(g, &g->hyb_rec, 2 * (size_t)g->m);
-      if (st) return st;
+    if (g->res_cluster == 0 && !g->hyb_rec && dalloc(g, &g->hyb_rec, 2 * (size_t)g->m)) {
+      g->hybrid = false;  // the persistent kernel needs no records
+      continue;
     }
     if (launch_ms) CK(cudaEventRecord(g->ev2, g->stream));
     ResParams p{};
@@ -2138,6 +2148,11 @@ PhaseBytes match_bytes(const wbpr_graph* g, const Stats& s, int64_t flow) {
 
 // ===========================================================================
 extern "C" {
+
+#ifdef WBPR_CHECKED
+// For tests of what a call does without the memory it asks for.
+void wbpr_checked_refuse_from(int64_t bytes) { wbpr::g_refuse_from = bytes; }
+#endif
 
 const char* wbpr_last_error(void) { return g_last_error.c_str(); }
 
