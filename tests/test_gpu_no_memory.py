@@ -46,3 +46,21 @@ for layout in ("bcsr", "rcsr"):
         refuse(0)
         assert d.solve("vc").flow == exact(g) and d.verify()["ok"] and d.device_bytes == held
 """)
+
+
+def test_cut_sides_without_any_room():
+    run(r"""
+for make in (lambda: W.gen_genrmf(6, 6, 1, 500, 2), lambda: W.gen_rmat(15, 8, seed=3)):
+    g = make()
+    _, sink, source = oracle.mincut(g.n, g.off, g.dst, g.cap, g.s, g.t)
+    tail = np.repeat(np.arange(g.n), np.diff(g.off))
+    for layout in ("bcsr", "rcsr"):
+        with W.DeviceGraph(g, layout) as d:
+            d.solve("vc")
+            refuse(1)
+            to_sink, from_source = d.cut_sides(0), d.cut_sides(1)
+            assert np.array_equal((to_sink[tail] == 0) & (to_sink[g.dst] == 1), sink != 0)
+            assert np.array_equal((from_source[tail] == 1) & (from_source[g.dst] == 0), source != 0)
+            refuse(0)
+            assert d.solve("vc").flow == exact(g) and d.verify()["ok"]
+""")

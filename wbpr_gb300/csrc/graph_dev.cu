@@ -165,7 +165,6 @@ struct wbpr_graph {
   int* cls = nullptr;
   int* vlab = nullptr;
   int8_t* ind = nullptr;
-  int8_t* sides = nullptr;
   int* flow_tmp = nullptr;
   long long* trace = nullptr;
   unsigned long long* bt = nullptr;
@@ -2675,11 +2674,12 @@ wbpr_status wbpr_cut_sides(wbpr_graph* g, int32_t side, int8_t* in_set) {
   if (st) return st;
   // n bytes to the host instead of 4 n and a loop over them: the whole call on
   // R-MAT, sink side, 144 -> 88 us at 131,072 vertices (RCSR), 604 -> 134 us
-  // at 1,048,576 (BCSR)
-  if (!g->sides && (st = dalloc(g, &g->sides, (size_t)g->n))) return st;
-  sides_kernel<<<std::min(g->sms * 4, (g->n + 255) / 256), 256, 0, g->stream>>>(g->vlab, g->n, g->sides);
+  // at 1,048,576 (BCSR).  The bytes lie in the relabel records, free between
+  // solves.
+  int8_t* sides = (int8_t*)g->rl_min;
+  sides_kernel<<<std::min(g->sms * 4, (g->n + 255) / 256), 256, 0, g->stream>>>(g->vlab, g->n, sides);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(in_set, g->sides, (size_t)g->n, cudaMemcpyDeviceToHost, g->stream));
+  CK(cudaMemcpyAsync(in_set, sides, (size_t)g->n, cudaMemcpyDeviceToHost, g->stream));
   CK(cudaStreamSynchronize(g->stream));
   return WBPR_OK;
 }
