@@ -64,3 +64,39 @@ for make in (lambda: W.gen_genrmf(6, 6, 1, 500, 2), lambda: W.gen_rmat(15, 8, se
             refuse(0)
             assert d.solve("vc").flow == exact(g) and d.verify()["ok"]
 """)
+
+
+def test_a_batch_without_room_for_arc_records():
+    run(r"""
+graphs = [W.gen_layered(31, 641, 3, 6, 1, 1000, 8), W.gen_grid(90, 80, 1), W.gen_genrmf(24, 20, 1, 10000, 5),
+          W.gen_genrmf(6, 9, 1, 10000, 2)]
+want = [exact(g) for g in graphs]
+with W.Batch(graphs) as b:
+    held = b.device_bytes
+    refuse(1)
+    assert b.solve()[0].tolist() == want and b.device_bytes == held
+    refuse(0)
+    assert b.solve(max_ms=60000.0)[0].tolist() == want and b.device_bytes > held  # another capture, with room
+""")
+
+
+def test_a_batch_holds_one_set_of_records():
+    """A split that asks for more records than the last one leaves only its own
+    behind.  (Four clusters of 16 blocks, or of one, hold four times the largest
+    instance's arcs; two and two hold less.)"""
+    run(r"""
+graphs = [W.gen_grid(100 + 10 * k, 90, k) for k in range(4)]
+want = [exact(g) for g in graphs]
+splits = (graphs[2].n + 2 * graphs[2].m, 1)  # from so many units on an instance has the largest cluster
+alone = []
+for c in splits:
+    with W.Batch(graphs) as one:
+        assert one.solve(batch_cluster=c)[0].tolist() == want
+        alone.append(one.device_bytes)
+assert alone[0] < alone[1]
+for order in (splits, splits[::-1]):
+    with W.Batch(graphs) as b:
+        for c in order:
+            assert b.solve(batch_cluster=c)[0].tolist() == want
+        assert b.device_bytes == alone[1], (b.device_bytes, alone)
+""")

@@ -369,6 +369,15 @@ wbpr_status balloc(wbpr_batch* b, T** p, size_t count) {
   return WBPR_OK;
 }
 
+// Gives back one array of balloc.
+template <class T>
+void bfree(wbpr_batch* b, T** p, size_t count) {
+  b->allocs.erase(std::find(b->allocs.begin(), b->allocs.end(), (void*)*p));
+  b->bytes -= (int64_t)(sizeof(T) * std::max<size_t>(count, 1));
+  cudaFreeAsync(*p, b->stream);
+  *p = nullptr;
+}
+
 void batch_release(wbpr_batch* b) {
   if (!b) return;
   cudaSetDevice(b->device);
@@ -461,38 +470,59 @@ wbpr_status capture(wbpr_batch* b, int tile, int block, double alpha, int grr, l
   static_assert(kLists == wbpr_batch::kLaunches, "one claim counter a launch");
   std::vector<int32_t> list[kLists];
   const int64_t big_units = cluster_units > 0 ? cluster_units : kBatchClusterUnits;
-  int hyb_most[kHybClasses] = {};  // clusters at once
-  int least = kHybClasses;    // the largest cluster there is
-  for (int k = kHybClasses - 1; k >= 0; --k) {
-    hyb_most[k] = mixed ? hybrid_clusters(kHybBlocks[k]) : 0;
-    if (hyb_most[k] == 0) break;
-    least = k;
-  }
-  std::vector<int32_t> hyb;
-  for (int32_t id : b->host_order) {
-    const wbpr_batch::Shape& x = b->shape[(size_t)id];
-    if (mixed && resident_one_block(x.n, x.arcs)) list[kResident].push_back(id);
-    else if (least < kHybClasses && hybrid_takes(x.n, x.arcs, x.longer) && hybrid_class(x.n, x.units(), 0, least) >= 0)
-      hyb.push_back(id);
-    else list[cluster_units >= 0 && x.units() >= big_units ? kCluster : kBlock].push_back(id);
-  }
-  // the shortest time in which the SMs can do the work that it asks for
-  auto class_of = [&](int32_t id, double t) {
-    const wbpr_batch::Shape& x = b->shape[(size_t)id];
-    if (cluster_units > 0) t = x.units() >= cluster_units ? 0 : 1e30;
-    return hybrid_class(x.n, x.units(), t, least);
-  };
-  double t = 1e5;
-  for (; t < 1e12; t *= 1.1) {
-    double ns = 0;  // SM x time
-    for (int32_t id : hyb) {
-      const int k = class_of(id, t);
-      ns += kHybMean * kHybNs[k] * kHybBlocks[k] * (double)b->shape[(size_t)id].units();
+  int hyb_clusters[kHybClasses];  // clusters at once
+  int64_t rec_first[kHybClasses], rec_stride[kHybClasses];  // their arc records
+  for (bool hybrid = mixed;; hybrid = false) {
+    int hyb_most[kHybClasses] = {};
+    int least = kHybClasses;  // the largest cluster there is
+    for (int k = kHybClasses - 1; k >= 0; --k) {
+      hyb_most[k] = hybrid ? hybrid_clusters(kHybBlocks[k]) : 0;
+      if (hyb_most[k] == 0) break;
+      least = k;
     }
-    for (int32_t id : list[kResident]) ns += kHybMean * kHybNs[kHybClasses - 1] * (double)b->shape[(size_t)id].units();
-    if (ns <= t * b->sms) break;
+    for (auto& l : list) l.clear();
+    std::vector<int32_t> hyb;
+    for (int32_t id : b->host_order) {
+      const wbpr_batch::Shape& x = b->shape[(size_t)id];
+      if (mixed && resident_one_block(x.n, x.arcs)) list[kResident].push_back(id);
+      else if (least < kHybClasses && hybrid_takes(x.n, x.arcs, x.longer) && hybrid_class(x.n, x.units(), 0, least) >= 0)
+        hyb.push_back(id);
+      else list[cluster_units >= 0 && x.units() >= big_units ? kCluster : kBlock].push_back(id);
+    }
+    // the shortest time in which the SMs can do the work that it asks for
+    auto class_of = [&](int32_t id, double t) {
+      const wbpr_batch::Shape& x = b->shape[(size_t)id];
+      if (cluster_units > 0) t = x.units() >= cluster_units ? 0 : 1e30;
+      return hybrid_class(x.n, x.units(), t, least);
+    };
+    double t = 1e5;
+    for (; t < 1e12; t *= 1.1) {
+      double ns = 0;  // SM x time
+      for (int32_t id : hyb) {
+        const int k = class_of(id, t);
+        ns += kHybMean * kHybNs[k] * kHybBlocks[k] * (double)b->shape[(size_t)id].units();
+      }
+      for (int32_t id : list[kResident]) ns += kHybMean * kHybNs[kHybClasses - 1] * (double)b->shape[(size_t)id].units();
+      if (ns <= t * b->sms) break;
+    }
+    for (int32_t id : hyb) list[kHybrid + class_of(id, t)].push_back(id);
+    int64_t rec_total = 0;
+    for (int k = 0; k < kHybClasses; ++k) {
+      rec_first[k] = rec_total;
+      rec_stride[k] = 0;
+      for (int32_t id : list[kHybrid + k]) rec_stride[k] = std::max(rec_stride[k], b->shape[(size_t)id].arcs);
+      hyb_clusters[k] = std::min((int)list[kHybrid + k].size(), hyb_most[k]);
+      rec_total += hyb_clusters[k] * rec_stride[k];
+    }
+    if (b->rec_count >= rec_total) break;
+    if (b->rec) bfree(b, &b->rec, (size_t)b->rec_count);  // every solve has been waited for
+    b->rec_count = 0;
+    if (balloc(b, &b->rec, (size_t)rec_total) == WBPR_OK) {
+      b->rec_count = rec_total;
+      break;
+    }
+    // no room for the records: without the hybrid solver
   }
-  for (int32_t id : hyb) list[kHybrid + class_of(id, t)].push_back(id);
   std::vector<int32_t> order;
   int first[kLists], count[kLists];
   for (int k = 0; k < kLists; ++k) {
@@ -502,22 +532,6 @@ wbpr_status capture(wbpr_batch* b, int tile, int block, double alpha, int grr, l
   }
   BCK(cudaMemcpyAsync(b->order, order.data(), 4 * order.size(), cudaMemcpyHostToDevice, b->stream));
   BCK(cudaStreamSynchronize(b->stream));
-  // arc records of the clusters that run at once
-  int64_t rec_first[kHybClasses], rec_stride[kHybClasses], rec_total = 0;
-  int hyb_clusters[kHybClasses];
-  for (int k = 0; k < kHybClasses; ++k) {
-    rec_first[k] = rec_total;
-    rec_stride[k] = 0;
-    for (int32_t id : list[kHybrid + k]) rec_stride[k] = std::max(rec_stride[k], b->shape[(size_t)id].arcs);
-    hyb_clusters[k] = std::min(count[kHybrid + k], hyb_most[k]);
-    rec_total += hyb_clusters[k] * rec_stride[k];
-  }
-  if (b->rec_count < rec_total) {
-    // (an earlier, smaller block stays with the batch until it is destroyed)
-    wbpr_status st = balloc(b, &b->rec, (size_t)rec_total);
-    if (st) return st;
-    b->rec_count = rec_total;
-  }
   const void* fn = kernel_for(tile, false);
   int occ = 0;
   BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, 0));
