@@ -554,13 +554,20 @@ __global__ void __launch_bounds__(kResThreads, 1) pr_resident_batch(const __grid
 
 }  // namespace
 
+bool resident_one_block(long long n, long long na) {
+  const long long slots = 32 * (n > kResThreads ? (n + 31) / 32 : kResThreads / 32);
+  return (long long)((sizeof(ResCtl) + 15) & ~15u) + kResArcBytes * na + kResVertexBytes * slots <= kResSmem && slots <= kResMaxVertices &&
+         na <= kResMaxArcs;
+}
+
 int resident_cluster(long long n, long long na) {
+  if (resident_one_block(n, na)) return 1;
+  // the blocks' shares are of equal weight, but for one row, and every block has
+  // a slot a thread, used or not
+  constexpr long long cs = kResMaxCluster, idle = kResVertexBytes * kResThreads;
   const long long w = kResVertexBytes * n + kResArcBytes * na;
-  // a block's share of a cluster may exceed the mean by one row
-  auto fits = [&](long long cs) {
-    return (cs == 1 ? w : w + w / 32) <= cs * (kResSmem - kResHeader) && n <= cs * kResMaxVertices && na <= cs * kResMaxArcs;
-  };
-  return fits(1) ? 1 : (fits(kResMaxCluster) ? kResMaxCluster : 0);
+  const long long share = (w + w / 32) / cs + (n < cs * kResThreads ? idle - kResVertexBytes * n / cs : 0);
+  return share <= kResSmem - kResHeader && n <= cs * kResMaxVertices && na <= cs * kResMaxArcs ? (int)cs : 0;
 }
 
 cudaError_t launch_resident(const ResParams& p0, int tile, int cluster, cudaStream_t st) {
@@ -569,12 +576,6 @@ cudaError_t launch_resident(const ResParams& p0, int tile, int cluster, cudaStre
   p.run.grp = cluster == 1 ? kResGrShareBlock : kResGrShare;
   if (cluster == 1) return tile < 32 ? launch_cluster<pr_resident<8, false>>(p, 1, st) : launch_cluster<pr_resident<32, false>>(p, 1, st);
   return tile < 32 ? launch_cluster<pr_resident<8, true>>(p, cluster, st) : launch_cluster<pr_resident<32, true>>(p, cluster, st);
-}
-
-bool resident_one_block(long long n, long long na) {
-  const long long slots = 32 * (n > kResThreads ? (n + 31) / 32 : kResThreads / 32);
-  return (long long)((sizeof(ResCtl) + 15) & ~15u) + kResArcBytes * na + kResVertexBytes * slots <= kResSmem && slots <= kResMaxVertices &&
-         na <= kResMaxArcs;
 }
 
 cudaError_t launch_resident_batch(const ResBatch& b0, int blocks, cudaStream_t st) {

@@ -129,8 +129,9 @@ cudaError_t launch_hybrid_batch(const ResBatch& b, int blocks, int clusters, cud
 // hybrid; layered 32x256 (80k) 0.52, 0.49; layered 64x512 (324k) 2.03, 1.10.
 constexpr long long kResPreferUnits = 1 << 17;
 
-// Cluster size for a graph of n vertices and na residual arcs: the smallest
-// power of two whose shared memory holds it, or 0.
+// Blocks for a graph of n vertices and na residual arcs: 1 where one block holds
+// it, kResMaxCluster where the cluster should (a row too long for its block's
+// share can still keep it out), or 0.
 int resident_cluster(long long n, long long na);
 cudaError_t launch_resident(const ResParams& p, int tile, int cluster, cudaStream_t st);
 // Whether one block holds the graph (exact).
