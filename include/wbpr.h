@@ -119,7 +119,11 @@ typedef struct wbpr_tuning {
                          /* left -> right, right -> t, every capacity 1, no other */
                          /* arc) is solved by the matching kernel; -1 = always    */
                          /* the general solver                                    */
-  int32_t pad2;
+  int32_t resident;      /* graphs that the shared-memory solvers take go to     */
+                         /* them: 0 = unless a knob of the persistent kernel is  */
+                         /* set (any of the above but max_rounds, max_ms, verify */
+                         /* and matching); 1 = whatever is set (but trace);      */
+                         /* -1 = never.  Single solves only                      */
   int64_t batch_cluster; /* batches: instances of at least this many units (n +   */
                          /* residual arcs) run on thread-block clusters, the rest */
                          /* one block each; 0 = every instance on the fewest      */
@@ -319,7 +323,9 @@ wbpr_status wbpr_solve_pairs(wbpr_graph* g, int32_t k, const int32_t* sources, c
  * {0.5, 1, 1.5, 3} and long-row thresholds {32, 64} on this graph and
  * these terminals (the faster of two solves each), then the best of those
  * with bfs_alpha 4, gr_plateau 4 and both; return the fastest tuning and its
- * solve time.  Every tuning must give the same flow (WBPR_ERR_VERIFY
+ * solve time.  On a graph that a shared-memory solver takes and solves faster
+ * than the persistent kernel does with the best of its knobs, the tuning
+ * returned has those knobs and resident = 1.  Every tuning must give the same flow (WBPR_ERR_VERIFY
  * otherwise).  The graph's state afterwards is that of the last solve. */
 wbpr_status wbpr_autotune(wbpr_graph* g, int32_t s, int32_t t, wbpr_algo algo, wbpr_tuning* best,
                           float* best_ms);

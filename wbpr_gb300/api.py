@@ -51,7 +51,7 @@ class Tuning(C.Structure):
                 ("gr_rounds", C.c_int32), ("grid_blocks", C.c_int32), ("gr_stall", C.c_int32),
                 ("barrier_timeout_ns", C.c_int64), ("greedy", C.c_int32), ("bfs_alpha", C.c_int32),
                 ("gr_plateau", C.c_int32), ("matching", C.c_int32),
-                ("pad2", C.c_int32), ("batch_cluster", C.c_int64)]
+                ("resident", C.c_int32), ("batch_cluster", C.c_int64)]
 
 
 class Result(C.Structure):
@@ -519,7 +519,8 @@ class DeviceGraph:
         return flows, r
 
     def autotune(self, algo="vc", s: int | None = None, t: int | None = None):
-        """(best Tuning, its solve ms) over tile, relabel frequency and long-row threshold."""
+        """(best Tuning, its solve ms) over tile, relabel frequency, long-row threshold and,
+        where one takes the graph, the shared-memory solver (resident = 1)."""
         tu = Tuning()
         ms = C.c_float(0)
         _check(lib().wbpr_autotune(self._h, -1 if s is None else s, -1 if t is None else t, ALGOS[algo],

@@ -1700,7 +1700,7 @@ struct RunCfg {
   int greedy;
   int bfs_alpha;
   int gr_plateau;
-  bool resident;  // no knob of the persistent kernel is set: the resident solver may take it
+  bool resident;  // the resident or the hybrid solver may take it
   bool matching;  // the matching kernel may take unit-capacity bipartite networks
   long long max_rounds;
   unsigned long long budget_ns;
@@ -2085,9 +2085,10 @@ wbpr_status make_cfg(wbpr_graph* g, int s, int t, wbpr_algo algo, const wbpr_tun
   const double ms = tu->max_ms > 0 ? tu->max_ms : 120000.0;
   rc->budget_ns = (unsigned long long)(ms * 1e6);
   rc->bfs_excl = -1;
-  rc->resident = !tu->tile && !tu->block && !tu->heavy_degree && !tu->blocks_per_sm && !tu->grid_blocks && !tu->trace &&
-                 alpha == kDefaultGrAlpha && !tu->gr_rounds && !tu->gr_stall && !tu->gr_plateau && !tu->bfs_alpha &&
-                 !tu->barrier_timeout_ns && !tu->greedy;
+  const bool knob = tu->tile || tu->block || tu->heavy_degree || tu->blocks_per_sm || tu->grid_blocks ||
+                    alpha != kDefaultGrAlpha || tu->gr_rounds || tu->gr_stall || tu->gr_plateau || tu->bfs_alpha ||
+                    tu->barrier_timeout_ns || tu->greedy;
+  rc->resident = !tu->trace && (tu->resident > 0 || (tu->resident == 0 && !knob));
   return WBPR_OK;
 }
 
@@ -2207,19 +2208,26 @@ wbpr_status wbpr_autotune(wbpr_graph* g, int32_t s, int32_t t, wbpr_algo algo, w
                           float* best_ms) {
   NvtxRange nvtx_("wbpr_autotune");
   if (!g || !best) return WBPR_ERR_INVALID_ARG;
+  // the defaults first.  A unit-capacity bipartite network goes to the matching
+  // kernel, which has none of the knobs below; the shared-memory solvers have
+  // none either, but the persistent kernel may still beat them.
+  float resident_ms = -1;  // the defaults' time where such a solver takes the graph
+  int64_t flow = -1;
   {
-    // a unit-capacity bipartite network goes to the matching kernel, which
-    // has none of the knobs below: the defaults, timed
     wbpr_tuning tu;
     wbpr_default_tuning(&tu);
     wbpr_result r0, r1;
     wbpr_status st = wbpr_solve(g, s, t, algo, &tu, &r0);
     if (st) return st;
-    if (r0.matching) {
+    flow = r0.flow;
+    if (r0.matching || g->res_cluster || g->hybrid) {
       if ((st = wbpr_solve(g, s, t, algo, &tu, &r1))) return st;
       if (r1.flow != r0.flow) return WBPR_ERR_VERIFY;
+      resident_ms = std::min(r0.solve_ms, r1.solve_ms);
+    }
+    if (r0.matching) {
       *best = tu;
-      if (best_ms) *best_ms = std::min(r0.solve_ms, r1.solve_ms);
+      if (best_ms) *best_ms = resident_ms;
       return WBPR_OK;
     }
   }
@@ -2231,7 +2239,6 @@ wbpr_status wbpr_autotune(wbpr_graph* g, int32_t s, int32_t t, wbpr_algo algo, w
   const int ntiles = algo == WBPR_ALGO_TC ? 1 : 3;
   float bms = 0;
   bool have = false;
-  int64_t flow = -1;
   for (int ti = 0; ti < ntiles; ++ti)
     for (double a : alphas)
       for (int hd : heavies) {
@@ -2245,8 +2252,7 @@ wbpr_status wbpr_autotune(wbpr_graph* g, int32_t s, int32_t t, wbpr_algo algo, w
           wbpr_result r;
           const wbpr_status st = wbpr_solve(g, s, t, algo, &tu, &r);
           if (st) return st;
-          if (flow >= 0 && r.flow != flow) return WBPR_ERR_VERIFY;  // every tuning must agree
-          flow = r.flow;
+          if (r.flow != flow) return WBPR_ERR_VERIFY;  // every tuning must agree
           ms = rep ? std::min(ms, r.solve_ms) : r.solve_ms;
         }
         if (!have || ms < bms) {
@@ -2275,6 +2281,10 @@ wbpr_status wbpr_autotune(wbpr_graph* g, int32_t s, int32_t t, wbpr_algo algo, w
       bms = ms;
       *best = tu;
     }
+  }
+  if (resident_ms >= 0 && resident_ms <= bms) {
+    bms = resident_ms;
+    best->resident = 1;
   }
   if (best_ms) *best_ms = bms;
   return WBPR_OK;
