@@ -178,24 +178,15 @@ __device__ bool setup(const ResInstance& in, char* sm, Part& P) {
 
 constexpr unsigned kBigRow = 128;  // rows longer than this are walked by a whole warp
 
-// Calls f(row j of the block, k) for the RCSR entries k of every row, forward
-// arcs first: 8 lanes a row, a warp for a long one (with 8 lanes there, R-MAT
-// scale 12 spent 0.13 ms of its 0.40 on loading its longest rows).
-template <class F>
-__device__ __forceinline__ void for_rows(const Part& P, F f) {
-  for (int j = threadIdx.x >> 3; j < P.nv; j += blockDim.x >> 3) {
-    const unsigned d = P.row[P.slot(j)] >> 16;
-    if (d <= kBigRow)
-      for (unsigned k = threadIdx.x & 7; k < d; k += 8) f(j, (int)k);
+// The row of entry x of n rows with offsets o: the last j with o[j] <= x.
+__device__ __forceinline__ int row_of_entry(const int* o, int n, int x) {
+  int lo = 0, hi = n;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (__ldg(o + mid) <= x) lo = mid;
+    else hi = mid;
   }
-  if (!P.big) return;
-  for (int j = threadIdx.x >> 5; j < P.nv; j += blockDim.x >> 5) {
-    const unsigned d = P.row[P.slot(j)] >> 16;
-    if (d > kBigRow) {
-#pragma unroll 4
-      for (unsigned k = threadIdx.x & 31; k < d; k += 32) f(j, (int)k);
-    }
-  }
+  return lo;
 }
 
 // Reads this block's rows (residuals from the capacities in a fresh solve).
@@ -229,25 +220,30 @@ __device__ void load(const ResInstance& in, Part& P) {
     return;
   }
   Sh<CL>::sync();  // every block's memory may be written from here on
-  for_rows(P, [&](int j, int k) {
-    const int v = v0 + j, fb = __ldg(in.frow + v), nf = __ldg(in.frow + v + 1) - fb;
-    const int here = (int)(P.row[P.slot(j)] & 0xffff) + k;
-    int2* q = P.rec + within(P.c, here, P.arcs);
+  // RCSR: a thread an entry, which finds its row by search.  (With 8 lanes a row
+  // and a warp for one over 128 arcs, a load waited for its longest rows: the sink
+  // side of the cut on R-MAT of 16 arcs a vertex, scale 10 0.283 -> 0.084 ms, scale
+  // 13 0.233 -> 0.098; the persistent kernel's search takes 0.074 and 0.091.)
+  const int f0 = __ldg(in.frow + v0), nf = __ldg(in.frow + v0 + P.nv) - f0, r0 = __ldg(in.rrow + v0);
+  for (int k = threadIdx.x; k < P.na; k += blockDim.x) {
     if (k < nf) {
-      int2 r = __ldcg(in.farc + fb + k);
+      const int f = f0 + k, v = v0 + row_of_entry(in.frow + v0, P.nv, f);
+      int2 r = __ldcg(in.farc + f);
       r.x = (int)within(P.c, r.x, P.n);
       const int o = owner_of(c, P.cs, r.x);
-      q->x = fresh ? __ldg(in.fcap + fb + k) : r.y;
+      int2* q = P.rec + within(P.c, f + __ldg(in.rrow + v) - a0, P.arcs);
+      q->x = fresh ? __ldg(in.fcap + f) : r.y;
       *(unsigned short*)&q->y = (unsigned short)(o << 12 | P.slot(r.x - c->bnd[o]));  // its twin is written below
     } else {
-      int2 r = __ldg(in.rarc + __ldg(in.rrow + v) + k - nf);  // {tail, forward arc}
+      const int e = r0 + k - nf, v = v0 + row_of_entry(in.rrow + v0, P.nv, e);
+      int2 r = __ldg(in.rarc + e);  // {tail, forward arc}
       r.x = (int)within(P.c, r.x, P.n);
-      const int o = owner_of(c, P.cs, r.x);
+      const int o = owner_of(c, P.cs, r.x), here = (int)within(P.c, e + __ldg(in.frow + v + 1) - a0, P.arcs);
       const unsigned tw = within(P.c, r.y + __ldg(in.rrow + r.x) - c->abase[o], P.arcs);
-      *q = make_int2(fresh ? 0 : __ldcg(in.fcb + r.y), (int)((unsigned)(o << 12 | P.slot(r.x - c->bnd[o])) | tw << 16));
+      P.rec[here] = make_int2(fresh ? 0 : __ldcg(in.fcb + r.y), (int)((unsigned)(o << 12 | P.slot(r.x - c->bnd[o])) | tw << 16));
       Sh<CL>::st16(Sh<CL>::at(P.a0, o) + P.a_rec + 8 * tw + 6, (unsigned)here);
     }
-  });
+  }
   Sh<CL>::sync();
 }
 
@@ -264,13 +260,13 @@ __device__ void write_back(const ResInstance& in, const Part& P) {
     for (int a = threadIdx.x; a < P.na; a += blockDim.x) in.arc[a0 + a].y = P.rec[a].x;
     return;
   }
-  for_rows(P, [&](int j, int k) {
-    const int f = __ldg(in.frow + v0 + j) + k;
-    if (f >= __ldg(in.frow + v0 + j + 1)) return;
-    const int cf = P.rec[(P.row[P.slot(j)] & 0xffff) + k].x;
+  const int f0 = __ldg(in.frow + v0), f1 = __ldg(in.frow + v0 + P.nv);
+  for (int f = f0 + threadIdx.x; f < f1; f += blockDim.x) {
+    const int v = v0 + row_of_entry(in.frow + v0, P.nv, f);
+    const int cf = P.rec[f + __ldg(in.rrow + v) - a0].x;
     in.farc[f].y = cf;
     in.fcb[f] = __ldg(in.fcap + f) - cf;
-  });
+  }
 }
 
 // Expands the vertices in slots u (one per W-lane tile, -1 for none) of label
