@@ -58,6 +58,7 @@ struct wbpr_batch {
   struct Shape {
     int64_t n, arcs;
     int64_t longer;  // rows of more than kLightDeg arcs
+    int64_t longest;  // arcs of the longest row but the terminals'
     int64_t units() const { return n + arcs; }
   };
   std::vector<Shape> shape;          // by instance
@@ -485,7 +486,8 @@ wbpr_status capture(wbpr_batch* b, int tile, int block, double alpha, int grr, l
     for (int32_t id : b->host_order) {
       const wbpr_batch::Shape& x = b->shape[(size_t)id];
       if (mixed && resident_one_block(x.n, x.arcs)) list[kResident].push_back(id);
-      else if (least < kHybClasses && hybrid_takes(x.n, x.arcs, x.longer) && hybrid_class(x.n, x.units(), 0, least) >= 0)
+      else if (least < kHybClasses && hybrid_takes(x.n, x.arcs, x.longer) && x.longest <= kHybLongRow &&
+               hybrid_class(x.n, x.units(), 0, least) >= 0)
         hyb.push_back(id);
       else list[cluster_units >= 0 && x.units() >= big_units ? kCluster : kBlock].push_back(id);
     }
@@ -749,9 +751,13 @@ wbpr_status wbpr_batch_create(const wbpr_csr* graphs, int32_t count, wbpr_batch*
       arx[2 * (ab + a) + 1] = r.arx[2 * a + 1];
     }
     inst[i] = BatchInst{(int)vb, n, (int)(vb + graphs[i].source), (int)(vb + graphs[i].sink)};
-    int64_t longer = 0;
-    for (int u = 0; u < n; ++u) longer += r.row[u + 1] - r.row[u] > kLightDeg;
-    b->shape[(size_t)i] = {n, na, longer};
+    int64_t longer = 0, longest = 0;
+    for (int u = 0; u < n; ++u) {
+      const int64_t d = r.row[u + 1] - r.row[u];
+      longer += d > kLightDeg;
+      if (u != graphs[i].source && u != graphs[i].sink) longest = std::max(longest, d);
+    }
+    b->shape[(size_t)i] = {n, na, longer, longest};
     vb += n;
     ab += na;
   }

@@ -194,6 +194,8 @@ struct wbpr_graph {
   // graph (0: none does), and what its launch reports
   int res_cluster = 0;
   bool hybrid = false;       // else the hybrid solver takes it, with one record an arc
+  // the three longest rows over kHeavyDeg arcs: arcs << 32 | vertex, longest first
+  unsigned long long longest[3] = {0, 0, 0};
   int4* hyb_rec = nullptr;
   ResOut* res_out = nullptr;
   int64_t bytes = 0;
@@ -1017,6 +1019,28 @@ __global__ void db_cls_scatter(const int* o1, const int* o2, int n, const int* s
     else cls[n01 + s2[u]] = u;
   }
 }
+// the three longest of nh heavy rows, arcs << 32 | vertex, longest first (0: none); one block
+__global__ void db_longest(const int* o1, const int* o2, const int* hcls, int nh, unsigned long long* out) {
+  __shared__ unsigned long long best;
+  unsigned long long below = ~0ull;
+  for (int k = 0; k < 3; ++k) {
+    if (threadIdx.x == 0) best = 0;
+    __syncthreads();
+    unsigned long long b = 0;
+    for (int j = threadIdx.x; j < nh; j += blockDim.x) {
+      const int u = hcls[j];
+      const unsigned long long x = (unsigned long long)(seg_len(o1, u) + seg_len(o2, u)) << 32 | (unsigned)u;
+      if (x < below && x > b) b = x;
+    }
+    if (b) atomicMax(&best, b);
+    __syncthreads();
+    below = best;
+    if (threadIdx.x == 0) out[k] = below;
+    if (below == 0) below = 1;  // none left: the other places are 0 too
+    __syncthreads();
+  }
+}
+
 // chunk items of heavy row j: kChunk pieces of each segment
 __global__ void db_heavy_chunks(const int* o1, const int* o2, const int* hcls, int nh, int* nch) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j <= nh; j += gridDim.x * blockDim.x) {
@@ -1432,6 +1456,11 @@ wbpr_status build_host(wbpr_graph* g, const wbpr_csr* in) {
   for (int u = 0; u < n; ++u) {
     const int d = length(u, 0) + length(u, 1);
     if (d > 0) cls[d <= kLightDeg ? 0 : (d <= kHeavyDeg ? 1 : 2)].push_back(u);
+    if (d > kHeavyDeg) {
+      unsigned long long x = (unsigned long long)d << 32 | (unsigned)u;
+      for (auto& y : g->longest)
+        if (x > y) std::swap(x, y);
+    }
     if (d > first) deep += (size_t)((d - first + kPart - 1) / kPart);
     if (d > kTdHeavy) {
       ++g->n_td_heavy;
@@ -1559,6 +1588,14 @@ wbpr_status build_on_device(wbpr_graph* g, const wbpr_csr* in) {
     CK(cudaMemsetAsync(g->ulog_n, 0, sizeof(int) * (size_t)kLogSlots * kLogStride, g->stream));
   }
   // in the stream the pool allocations were made on (stream-ordered memory)
+  if (g->n_heavy > 0 && g->n + g->total_deg <= kHybMaxUnits) {  // a graph that a shared-memory solver may take
+    auto* three = (unsigned long long*)g->h;  // 64 words at least, cleared below
+    const bool bcsr = g->layout == WBPR_LAYOUT_BCSR;
+    db_longest<<<1, 256, 0, g->stream>>>(bcsr ? g->row : g->frow, bcsr ? nullptr : g->rrow, g->cls + g->n_light + g->n_medium,
+                                         g->n_heavy, three);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(g->longest, three, sizeof(g->longest), cudaMemcpyDeviceToHost, g->stream));
+  }
   CK(cudaMemsetAsync(g->h, 0, 4 * (size_t)g->n, g->stream));
   CK(cudaMemsetAsync(g->e, 0, 4 * (size_t)g->n, g->stream));
   CK(cudaStreamSynchronize(g->stream));
@@ -1701,6 +1738,7 @@ struct RunCfg {
   int bfs_alpha;
   int gr_plateau;
   bool resident;  // the resident or the hybrid solver may take it
+  bool phase2;    // kModeState: return_stranded()
   bool matching;  // the matching kernel may take unit-capacity bipartite networks
   long long max_rounds;
   unsigned long long budget_ns;
@@ -1801,8 +1839,19 @@ wbpr_status run_kernel(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch
   return WBPR_OK;
 }
 
+// The longest row over kHeavyDeg arcs that is neither of the two vertices', or 0.
+long long long_row(const wbpr_graph* g, int s, int t) {
+  for (unsigned long long x : g->longest)
+    if ((int)(x & 0xffffffffu) != s && (int)(x & 0xffffffffu) != t) return (long long)(x >> 32);
+  return 0;
+}
+
+// Whether a launch goes to the resident or the hybrid solver.
 bool use_resident(const wbpr_graph* g, const RunCfg& rc) {
-  return rc.resident && !rc.term && (g->res_cluster > 0 || g->hybrid);
+  if (!rc.resident || rc.term || (g->res_cluster == 0 && !g->hybrid)) return false;
+  const bool search = rc.mode == kModeBfsOnly || rc.phase2;
+  const long long row = long_row(g, rc.s, rc.t);
+  return row <= (g->res_cluster ? (search ? kResLongSearch : kResLongRow) : (search ? kHybLongSearch : kHybLongRow));
 }
 
 // One launch of the resident or the hybrid solver.  *fits is cleared when
@@ -2220,7 +2269,9 @@ wbpr_status wbpr_autotune(wbpr_graph* g, int32_t s, int32_t t, wbpr_algo algo, w
     wbpr_status st = wbpr_solve(g, s, t, algo, &tu, &r0);
     if (st) return st;
     flow = r0.flow;
-    if (r0.matching || g->res_cluster || g->hybrid) {
+    RunCfg rc;
+    if ((st = make_cfg(g, s < 0 ? g->s : s, t < 0 ? g->t : t, algo, &tu, &rc))) return st;
+    if (r0.matching || use_resident(g, rc)) {
       if ((st = wbpr_solve(g, s, t, algo, &tu, &r1))) return st;
       if (r1.flow != r0.flow) return WBPR_ERR_VERIFY;
       resident_ms = std::min(r0.solve_ms, r1.solve_ms);
@@ -2649,6 +2700,7 @@ static wbpr_status return_stranded(wbpr_graph* g) {
   wbpr_status st = make_cfg(g, g->t, g->s, WBPR_ALGO_VC, nullptr, &rc);
   if (st) return st;
   rc.mode = kModeState;
+  rc.phase2 = true;
   rc.bfs_excl = g->t;
   Stats hs;
   return run(g, rc, &hs);

@@ -84,7 +84,8 @@ __global__ void na_reset(int2* arc, const int2* arx, long long na) {
 // counts: [0] light, [1] medium, [2] heavy, [3] long-row chunks,
 //         [4..7] fill cursors of the second pass, [8] malformed rows,
 //         [9] malformed arcs, [10] vertices whose incoming capacity passes int32,
-//         [11] arcs whose twin lies outside their head's row
+//         [11] what keeps the graph off the resident solver: arcs whose twin
+//         lies outside their head's row, rows that are too long for it
 __global__ void na_count(const int* row, int n, long long na, int* counts) {
   if (blockIdx.x == 0 && threadIdx.x == 0 && (row[0] != 0 || (long long)row[n] != na)) atomicAdd(counts + 8, 1);
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
@@ -174,12 +175,15 @@ __global__ void na_check_heavy(const int* cls, int first, int nh, const unsigned
 // takes: one thread an arc, which finds its row by binary search (a malformed
 // row array only makes it find a wrong row) and adds its twin's capacity to the
 // row's sum; na_check_sums reads the sums.
-__global__ void na_check_all(const int* row, const int2* arc, const int2* arx, int n, long long na,
+__global__ void na_check_all(const int* row, const int2* arc, const int2* arx, int n, long long na, int s, int t,
                              unsigned long long* insum, int* counts) {
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
   if (gt == 0 && (row[0] != 0 || (long long)row[n] != na)) atomicAdd(counts + 8, 1);
-  for (int v = gt; v < n; v += gs)
-    if (row[v + 1] < row[v]) atomicAdd(counts + 8, 1);
+  for (int v = gt; v < n; v += gs) {
+    const long long d = (long long)row[v + 1] - row[v];
+    if (d < 0) atomicAdd(counts + 8, 1);
+    if (d > kResLongRow && v != s && v != t) atomicAdd(counts + 11, 1);
+  }
   int bad = 0;
   for (int a = gt; a < (int)na; a += gs) {
     const int2 r = arc[a], x = arx[a];
@@ -267,6 +271,7 @@ extern "C" wbpr_status wbpr_solve_bcsr_noalloc(int32_t n, int64_t num_residual_a
   const int2* arx = (const int2*)d_arx;
   int* vert = base + kOffVert;
   auto va = [&](int i) { return vert + (long long)i * kNoAllocMaxVertices; };
+  bool checked = false;
   // A graph that fits the resident solver: the checks, then the solve, which
   // does nothing when they found something, and one wait for both (R-MAT scale
   // 13 0.66 -> 0.50 ms).
@@ -279,7 +284,7 @@ extern "C" wbpr_status wbpr_solve_bcsr_noalloc(int32_t n, int64_t num_residual_a
       int counts[12];
     } h;
     NA_CK(cudaMemsetAsync(insum, 0, sizeof(unsigned long long) * (size_t)n, st));
-    na_check_all<<<sms * 2, 256, 0, st>>>(d_row, arc, arx, n, num_residual_arcs, insum, counts);
+    na_check_all<<<sms * 2, 256, 0, st>>>(d_row, arc, arx, n, num_residual_arcs, s, t, insum, counts);
     na_check_sums<<<(n + 255) / 256, 256, 0, st>>>(insum, n, counts);
     NA_CK(cudaGetLastError());
     ResParams rp{};
@@ -310,6 +315,7 @@ extern "C" wbpr_status wbpr_solve_bcsr_noalloc(int32_t n, int64_t num_residual_a
       *flow = h.out.flow;
       return WBPR_OK;
     }
+    checked = true;
     NA_CK(cudaMemsetAsync(counts, 0, sizeof(int) * kCountWords, st));
   }
   int* cls = va(14);
@@ -324,17 +330,19 @@ extern "C" wbpr_status wbpr_solve_bcsr_noalloc(int32_t n, int64_t num_residual_a
   NA_CK(cudaStreamSynchronize(st));
   if (wbpr_status bad = refuse(hc)) return bad;
   na_fill<<<sms * 2, 256, 0, st>>>(d_row, n, counts, cls, bch);
-  // the per-vertex incoming-capacity sums borrow two vertex arrays (active
-  // lists the solver fills before it reads them)
-  unsigned long long* insum = (unsigned long long*)va(4);
-  NA_CK(cudaMemsetAsync(insum, 0, sizeof(unsigned long long) * (size_t)n, st));
-  na_check<<<sms * 2, 256, 0, st>>>(d_row, arc, arx, n, num_residual_arcs, cls, hc[0] + hc[1], bch, hc[3], insum,
-                                    counts);
-  na_check_heavy<<<sms, 256, 0, st>>>(cls, hc[0] + hc[1], hc[2], insum, counts);
-  NA_CK(cudaGetLastError());
-  NA_CK(cudaMemcpyAsync(hc, counts, sizeof(hc), cudaMemcpyDeviceToHost, st));
-  NA_CK(cudaStreamSynchronize(st));
-  if (wbpr_status bad = refuse(hc)) return bad;
+  if (!checked) {
+    // the per-vertex incoming-capacity sums borrow two vertex arrays (active
+    // lists the solver fills before it reads them)
+    auto* insum = (unsigned long long*)va(4);
+    NA_CK(cudaMemsetAsync(insum, 0, sizeof(unsigned long long) * (size_t)n, st));
+    na_check<<<sms * 2, 256, 0, st>>>(d_row, arc, arx, n, num_residual_arcs, cls, hc[0] + hc[1], bch, hc[3], insum,
+                                      counts);
+    na_check_heavy<<<sms, 256, 0, st>>>(cls, hc[0] + hc[1], hc[2], insum, counts);
+    NA_CK(cudaGetLastError());
+    NA_CK(cudaMemcpyAsync(hc, counts, sizeof(hc), cudaMemcpyDeviceToHost, st));
+    NA_CK(cudaStreamSynchronize(st));
+    if (wbpr_status bad = refuse(hc)) return bad;
+  }
   if (num_residual_arcs > 0) na_reset<<<sms * 4, 256, 0, st>>>(arc, arx, num_residual_arcs);
 
   Params<TopoB> p{};  // every field zero unless it has its own initializer

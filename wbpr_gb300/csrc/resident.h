@@ -129,6 +129,24 @@ cudaError_t launch_hybrid_batch(const ResBatch& b, int blocks, int clusters, cud
 // hybrid; layered 32x256 (80k) 0.52, 0.49; layered 64x512 (324k) 2.03, 1.10.
 constexpr long long kResPreferUnits = 1 << 17;
 
+// The shared-memory solvers walk a row with one warp (resident) or 8 lanes
+// (hybrid), the persistent kernel a long one with the whole grid: graphs that
+// have a longer row than this, other than a terminal's, are the persistent
+// kernel's.  Solves, persistent and shared-memory, one row of so many arcs:
+// resident (s -> hub -> d rays -> t) 4,000 0.46, 0.31 ms, 7,000 0.50, 0.43,
+// 10,000 0.44, 0.60, 20,000 0.47, 1.15; hybrid (random graphs of 12,000 to
+// 120,000 vertices) 4,000 2.2, 1.2; 2.3, 1.4; 2.4, 1.3; 1.3, 1.0 ms, 8,000 2.0,
+// 1.2; 2.7, 1.8; 2.6, 1.9; 0.7, 1.2, 16,000 1.3, 3.3; 2.1, 3.2; 1.5, 3.1; 0.6,
+// 1.8; rays of 29,000 0.47, 6.8, in batches of 8 12,000 1 16,000 5.4, 6.4.
+constexpr int kResLongRow = 8192;
+constexpr int kHybLongRow = 4096;
+// The same for a search alone, and phase 2, whose first search is most of it:
+// resident 4,000 rays 0.08, 0.08 ms and 0.14, 0.12, 7,000 0.08, 0.11 and 0.14,
+// 0.15; hybrid 2,000 0.21, 0.18 and 0.17, 0.16, 4,000 0.22, 0.23 and 0.18, 0.21,
+// 8,000 0.32, 0.39 and 0.26, 0.47.
+constexpr int kResLongSearch = 4096;
+constexpr int kHybLongSearch = 2048;
+
 // Blocks for a graph of n vertices and na residual arcs: 1 where one block holds
 // it, kResMaxCluster where the cluster should (a row too long for its block's
 // share can still keep it out), or 0.
