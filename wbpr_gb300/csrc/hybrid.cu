@@ -241,21 +241,13 @@ struct List {
       n += __popc(m);
     }
   }
-  // calls f(slot, word) for all of them, 32 / W at once (-1, 0 for a tile
-  // without one): word is the slot's of the array at `words` (0: no array).
-  // A lane reads 32 of them at a time, one each.
+  // calls f(slot) for all of them, 32 / W at once (-1 for a tile without one)
   template <int W, class F>
-  __device__ __forceinline__ void drain(unsigned words, F f) {
+  __device__ __forceinline__ void drain(F f) {
     __syncwarp();
-    for (int i = 0; i < n; i += 32) {
-      const int lane = threadIdx.x & 31;
-      int u = -1, x = 0;
-      if (i + lane < n) {
-        u = (int)lds16(at + 2 * (i + lane));
-        if (words) x = (int)lds32(words + 4 * u);
-      }
-      for (int k = 0; k < 32 && i + k < n; k += 32 / W)
-        f(__shfl_sync(kFull, u, k + lane / W), words ? __shfl_sync(kFull, x, k + lane / W) : 0);
+    for (int i = 0; i < n; i += 32 / W) {
+      const int k = i + (threadIdx.x & 31) / W;
+      f(k < n ? (int)lds16(at + 2 * k) : -1);
     }
     __syncwarp();
     n = 0;
@@ -307,7 +299,7 @@ __device__ int bfs_hybrid(const ResParams& p, const HPart& P, int& seq, Count& c
     bool did = false;
     for (int k = 0; k < p.run.bsub; ++k) {
       bool now = false;
-      const auto expand = [&](int u, int) { bfs_expand<kTile, DIR>(in, P, u, ct); };
+      const auto expand = [&](int u) { bfs_expand<kTile, DIR>(in, P, u, ct); };
       for (int g = wid; g < P.groups; g += nw) {
         const unsigned at = 512 * g + 16 * lane;
         const int4 l = lds128(P.a0 + P.a_lab + at), x = lds128(P.a0 + P.a_ex + at);
@@ -317,9 +309,9 @@ __device__ int bfs_hybrid(const ResParams& p, const HPart& P, int& seq, Count& c
         if (open)
           sts128(P.a0 + P.a_ex + at, make_int4(min(l.x, x.x), min(l.y, x.y), min(l.z, x.z), min(l.w, x.w)));
         list.add(g, open);
-        if (list.n > 128) list.drain<kTile>(0, expand);
+        if (list.n > 128) list.drain<kTile>(expand);
       }
-      list.drain<kTile>(0, expand);
+      list.drain<kTile>(expand);
       did |= now;
       if (k + 1 < p.run.bsub && !__syncthreads_or(now)) break;
     }
@@ -331,15 +323,17 @@ __device__ int bfs_hybrid(const ResParams& p, const HPart& P, int& seq, Count& c
 // Push and relabel, as discharge() of the resident solver (the same argument
 // keeps the labels valid, and E is what one lane read); pushes into t are summed by the thread.
 template <int W>
-__device__ __forceinline__ void discharge(const ResInstance& in, const HPart& P, int u, int E, int& sink, Count& ct) {
+__device__ __forceinline__ void discharge(const ResInstance& in, const HPart& P, int u, int& sink, Count& ct) {
   const int lane = threadIdx.x & (W - 1);
   lanes_apart();
-  int hu = 0;  // no other warp writes it
+  int E = 0, hu = 0;  // (no other warp writes the label)
   int2 row = make_int2(0, 0);
   if (u >= 0) {
+    if (lane == 0) E = (int)lds32(P.a0 + P.a_e + 4 * u);
     hu = (int)lds32(P.a0 + P.a_lab + 4 * u);
     row = row_of(in, P, u);
   }
+  E = __shfl_sync(kFull, E, 0, W);
   unsigned erem = (unsigned)E;
   int mn = kBig, k = 0;
   constexpr int Q = 2;
@@ -415,7 +409,7 @@ __device__ bool push_step(const ResInstance& in, const HPart& P, Count& ct) {
   bool did = false;
   int sink = 0;
   List list(P);
-  const auto work = [&](int u, int E) { discharge<kTile>(in, P, u, E, sink, ct); };
+  const auto work = [&](int u) { discharge<kTile>(in, P, u, sink, ct); };
   for (int g = wid; g < P.groups; g += nw) {
     const unsigned at = 512 * g + 16 * lane;
     const int4 e = lds128(P.a0 + P.a_e + at);
@@ -425,9 +419,9 @@ __device__ bool push_step(const ResInstance& in, const HPart& P, Count& ct) {
     if (P.tl >> 2 == 32 * g + lane) act &= ~(1u << (P.tl & 3));
     list.add(g, act);
     did |= list.n > 0;
-    if (list.n > 128) list.drain<kTile>(P.a0 + P.a_e, work);
+    if (list.n > 128) list.drain<kTile>(work);
   }
-  list.drain<kTile>(P.a0 + P.a_e, work);
+  list.drain<kTile>(work);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sink += __shfl_xor_sync(kFull, sink, o);
   if (lane == 0 && sink) Smem::add(Smem::at(P.a0, (unsigned)P.tv >> 16) + P.a_e + 4 * (P.tv & 0xffff), sink);
