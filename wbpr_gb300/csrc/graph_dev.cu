@@ -1588,7 +1588,8 @@ wbpr_status build_on_device(wbpr_graph* g, const wbpr_csr* in) {
     CK(cudaMemsetAsync(g->ulog_n, 0, sizeof(int) * (size_t)kLogSlots * kLogStride, g->stream));
   }
   // in the stream the pool allocations were made on (stream-ordered memory)
-  if (g->n_heavy > 0 && g->n + g->total_deg <= kHybMaxUnits) {  // a graph that a shared-memory solver may take
+  // a graph that a shared-memory solver may take, or one with few long rows
+  if (g->n_heavy > 0 && (g->n + g->total_deg <= kHybMaxUnits || g->n_td_heavy < kFewLong)) {
     auto* three = (unsigned long long*)g->h;  // 64 words at least, cleared below
     const bool bcsr = g->layout == WBPR_LAYOUT_BCSR;
     db_longest<<<1, 256, 0, g->stream>>>(bcsr ? g->row : g->frow, bcsr ? nullptr : g->rrow, g->cls + g->n_light + g->n_medium,
@@ -1769,6 +1770,13 @@ wbpr_status ensure_trace(wbpr_graph* g) {
   return WBPR_OK;
 }
 
+// The longest row over kHeavyDeg arcs that is neither of the two vertices', or 0.
+long long long_row(const wbpr_graph* g, int s, int t) {
+  for (unsigned long long x : g->longest)
+    if ((int)(x & 0xffffffffu) != s && (int)(x & 0xffffffffu) != t) return (long long)(x >> 32);
+  return 0;
+}
+
 template <class Topo>
 wbpr_status run_kernel(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch_ms) {
   Params<Topo> p{};  // every field zero unless it has its own initializer
@@ -1778,7 +1786,7 @@ wbpr_status run_kernel(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch
   p.t = rc.t;
   p.mode = rc.mode;
   p.heavy_deg = rc.heavy_deg;
-  p.first = first_arcs((long long)g->n + g->total_deg);
+  p.first = first_arcs((long long)g->n + g->total_deg, !rc.term && g->n_td_heavy < kFewLong && long_row(g, rc.s, rc.t) == 0);
   p.gr_threshold = rc.gr_threshold;
   p.gr_rounds = rc.gr_rounds;
   p.gr_stall = rc.gr_stall;
@@ -1837,13 +1845,6 @@ wbpr_status run_kernel(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch
     return WBPR_ERR_VERIFY;
   }
   return WBPR_OK;
-}
-
-// The longest row over kHeavyDeg arcs that is neither of the two vertices', or 0.
-long long long_row(const wbpr_graph* g, int s, int t) {
-  for (unsigned long long x : g->longest)
-    if ((int)(x & 0xffffffffu) != s && (int)(x & 0xffffffffu) != t) return (long long)(x >> 32);
-  return 0;
 }
 
 // Whether a launch goes to the resident or the hybrid solver.

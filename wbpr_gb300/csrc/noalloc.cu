@@ -85,13 +85,18 @@ __global__ void na_reset(int2* arc, const int2* arx, long long na) {
 //         [4..7] fill cursors of the second pass, [8] malformed rows,
 //         [9] malformed arcs, [10] vertices whose incoming capacity passes int32,
 //         [11] what keeps the graph off the resident solver: arcs whose twin
-//         lies outside their head's row, rows that are too long for it
-__global__ void na_count(const int* row, int n, long long na, int* counts) {
+//         lies outside their head's row, rows that are too long for it;
+//         rows but the terminals': [12] over kTdHeavy arcs, [13] over kHeavyDeg
+__global__ void na_count(const int* row, int n, long long na, int s, int t, int* counts) {
   if (blockIdx.x == 0 && threadIdx.x == 0 && (row[0] != 0 || (long long)row[n] != na)) atomicAdd(counts + 8, 1);
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
     const int d = row[v + 1] - row[v];
     if (d < 0) atomicAdd(counts + 8, 1);
     if (d <= 0) continue;
+    if (d > kTdHeavy && v != s && v != t) {
+      atomicAdd(counts + 12, 1);
+      if (d > kHeavyDeg) atomicAdd(counts + 13, 1);
+    }
     if (d <= kLightDeg) atomicAdd(counts + 0, 1);
     else if (d <= kHeavyDeg) atomicAdd(counts + 1, 1);
     else {
@@ -323,9 +328,9 @@ extern "C" wbpr_status wbpr_solve_bcsr_noalloc(int32_t n, int64_t num_residual_a
   // The rows are checked before anything sizes work by them: the class list
   // and the chunk items are bounded by the declared arc count only when
   // row[0] == 0, row[n] == num_residual_arcs and no row is negative.
-  na_count<<<sms * 2, 256, 0, st>>>(d_row, n, num_residual_arcs, counts);
+  na_count<<<sms * 2, 256, 0, st>>>(d_row, n, num_residual_arcs, s, t, counts);
   NA_CK(cudaGetLastError());
-  int hc[11];
+  int hc[14];
   NA_CK(cudaMemcpyAsync(hc, counts, sizeof(hc), cudaMemcpyDeviceToHost, st));
   NA_CK(cudaStreamSynchronize(st));
   if (wbpr_status bad = refuse(hc)) return bad;
@@ -390,7 +395,7 @@ extern "C" wbpr_status wbpr_solve_bcsr_noalloc(int32_t n, int64_t num_residual_a
   p.budget_ns = 120ull * 1000 * 1000 * 1000;
   p.bar_timeout_ns = 10ull * 1000 * 1000 * 1000;
   p.heavy_deg = 32;
-  p.first = first_arcs((long long)n + num_residual_arcs);
+  p.first = first_arcs((long long)n + num_residual_arcs, hc[12] < kFewLong && hc[13] == 0);
   p.mode = kModeFresh;
   p.bfs_excl = s;
   const int tile = algo == WBPR_ALGO_TC ? 1 : 32;

@@ -569,7 +569,15 @@ __device__ __forceinline__ void vidx(const VRow& r, int vi, int& k, int& a) {
 // 1.03, 1.00, 17 (2.8M units) 1.07, 1.02, 18 (8.1M units) 1.05, 1.06; RCSR 0.91,
 // 0.88, 1.10, 1.08, 1.14, 1.09, 1.05, 1.07.
 constexpr long long kFirstUnits[3] = {1LL << 22, 1LL << 24, 100000000};  // n + residual arcs, for 128, 256 and 512 arcs
-inline int first_arcs(long long units) {
+// Where few rows are long at all, and none but a terminal's over 2,048 arcs,
+// nothing goes deep: the two deep passes and their barriers in every round cost
+// more than the one or two warps that walk on.  At 2,048 and 128 arcs: random
+// graphs of 60,000 vertices with one row of 2,000 1.11, 1.16 ms (RCSR 1.26,
+// 1.32), with four of 1,000 2.28, 2.41 (2.44, 2.54), a 220x220 grid with one of
+// 600 7.7, 8.0 (8.1, 8.5); with one of 16,000 2.37, 2.19 (2.52, 2.15).
+constexpr int kFewLong = 32;  // rows over kTdHeavy arcs
+inline int first_arcs(long long units, bool few_long = false) {
+  if (few_long) return 2048;
   return units <= kFirstUnits[0] ? 128 : (units <= kFirstUnits[1] ? 256 : (units <= kFirstUnits[2] ? 512 : 2048));
 }
 constexpr int kPart = 256;               // arcs of a deep part: one warp, 8 arcs a lane in flight
