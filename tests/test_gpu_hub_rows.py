@@ -50,7 +50,7 @@ def test_a_hub_goes_to_the_persistent_kernel(rays, layout):
 
 
 def test_a_batch_of_hubs_goes_to_the_general_kernel():
-    graphs = [_rays(5000, k) for k in range(8)]
+    graphs = [_rays(10000, k) for k in range(8)]
     want = [oracle.dinic(g.n, g.off, g.dst, g.cap, g.s, g.t) for g in graphs]
     with W.Batch(graphs) as b:
         assert b.solve()[0].tolist() == want

@@ -197,6 +197,7 @@ struct wbpr_graph {
   // the three longest rows over kHeavyDeg arcs: arcs << 32 | vertex, longest first
   unsigned long long longest[3] = {0, 0, 0};
   int4* hyb_rec = nullptr;
+  int levels = 0;                 // of a search in the last solve, on average
   ResOut* res_out = nullptr;
   int64_t bytes = 0;
   std::vector<void*> allocs;
@@ -1851,8 +1852,13 @@ wbpr_status run_kernel(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch
 bool use_resident(const wbpr_graph* g, const RunCfg& rc) {
   if (!rc.resident || rc.term || (g->res_cluster == 0 && !g->hybrid)) return false;
   const bool search = rc.mode == kModeBfsOnly || rc.phase2;
+  const long long units = g->n + g->total_deg;
+  if (search && g->res_cluster > 1 && g->avg_deg >= kResDenseDegree && units > kResDenseUnits) return false;
+  if (rc.mode == kModeBfsOnly && !g->res_cluster && units > kHybShallowUnits && g->levels < kHybShallowLevels) return false;
   const long long row = long_row(g, rc.s, rc.t);
-  return row <= (g->res_cluster ? (search ? kResLongSearch : kResLongRow) : (search ? kHybLongSearch : kHybLongRow));
+  if (g->res_cluster) return row <= (search ? kResLongSearch : kResLongRow);
+  if (search && g->levels < kHybShallowLevels) return row <= kHybLongSearch;
+  return row <= (units > kHybLargeUnits ? kHybLongRowLarge : kHybLongRow);
 }
 
 // One launch of the resident or the hybrid solver.  *fits is cleared when
@@ -1922,14 +1928,18 @@ wbpr_status run_resident(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* laun
   return (wbpr_status)h.err;
 }
 
+wbpr_status run_persistent(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch_ms) {
+  return g->layout == WBPR_LAYOUT_RCSR ? run_kernel<TopoR>(g, rc, hs, launch_ms)
+                                       : run_kernel<TopoB>(g, rc, hs, launch_ms);
+}
+
 wbpr_status run(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch_ms = nullptr) {
-  if (rc.mode != kModeFresh && use_resident(g, rc)) {
+  if (rc.mode != kModeFresh && use_resident(g, rc)) {  // (a fresh solve has asked already)
     bool fits = false;
     const wbpr_status st = run_resident(g, rc, hs, launch_ms, nullptr, &fits);
     if (st || fits) return st;
   }
-  return g->layout == WBPR_LAYOUT_RCSR ? run_kernel<TopoR>(g, rc, hs, launch_ms)
-                                       : run_kernel<TopoB>(g, rc, hs, launch_ms);
+  return run_persistent(g, rc, hs, launch_ms);
 }
 
 // Rows longer than this are discharged by a whole warp in the matching kernel
@@ -2464,6 +2474,7 @@ wbpr_status wbpr_solve(wbpr_graph* g, int32_t s, int32_t t, wbpr_algo algo, cons
   CK(cudaEventSynchronize(g->ev1));
   if (st) return st;
   if (!done) CK(cudaMemcpy(&et, g->e + t, 4, cudaMemcpyDeviceToHost));
+  g->levels = hs.bfs_levels / std::max(1, hs.grs);
   if (out) {
     std::memset(out, 0, sizeof(*out));
     out->flow = et;

@@ -134,18 +134,41 @@ constexpr long long kResPreferUnits = 1 << 17;
 // have a longer row than this, other than a terminal's, are the persistent
 // kernel's.  Solves, persistent and shared-memory, one row of so many arcs:
 // resident (s -> hub -> d rays -> t) 4,000 0.46, 0.31 ms, 7,000 0.50, 0.43,
-// 10,000 0.44, 0.60, 20,000 0.47, 1.15; hybrid (random graphs of 12,000 to
-// 120,000 vertices) 4,000 2.2, 1.2; 2.3, 1.4; 2.4, 1.3; 1.3, 1.0 ms, 8,000 2.0,
-// 1.2; 2.7, 1.8; 2.6, 1.9; 0.7, 1.2, 16,000 1.3, 3.3; 2.1, 3.2; 1.5, 3.1; 0.6,
-// 1.8; rays of 29,000 0.47, 6.8, in batches of 8 12,000 1 16,000 5.4, 6.4.
+// 10,000 0.44, 0.60, 20,000 0.47, 1.15; hybrid (random graphs of 164k to 692k
+// units) 4,000 2.2, 1.2; 2.3, 1.4; 2.4, 1.3 ms, 8,000 2.0, 1.2; 2.7, 1.8; 2.6, 1.9,
+// 16,000 1.3, 3.3; 2.1, 3.2; 1.5, 3.1; of 1.1M 4,000 1.3, 1.0, 8,000 0.7, 1.2;
+// rays of 29,000 0.47, 6.8.  Batches of 8, general kernel and hybrid: 8,000 3.9,
+// 2.4; 7.9, 4.8, 16,000 5.4, 6.4; 7.9, 5.8, rays of 10,000 2.8, 4.7.
 constexpr int kResLongRow = 8192;
-constexpr int kHybLongRow = 4096;
-// The same for a search alone, and phase 2, whose first search is most of it:
-// resident 4,000 rays 0.08, 0.08 ms and 0.14, 0.12, 7,000 0.08, 0.11 and 0.14,
-// 0.15; hybrid 2,000 0.21, 0.18 and 0.17, 0.16, 4,000 0.22, 0.23 and 0.18, 0.21,
-// 8,000 0.32, 0.39 and 0.26, 0.47.
+constexpr int kHybLongRow = 8192;
+constexpr int kHybLongRowLarge = 4096;  // above kHybLargeUnits
+constexpr long long kHybLargeUnits = 1 << 20;
+// The same for phase 2 and a search alone (the hybrid's only where the last
+// solve's searches had fewer than kHybShallowLevels levels: in deeper ones a row is
+// one step of many).  Resident, 4,000 rays 0.14, 0.12 ms and 0.08, 0.08, 7,000 0.14,
+// 0.15 and 0.08, 0.11; hybrid, random graphs 2,000 0.17, 0.16 and 0.21, 0.18, 4,000
+// 0.18, 0.21 and 0.22, 0.23, 8,000 0.26, 0.47 and 0.32, 0.39, a 220x220 grid with a
+// row of 2,400 0.41, 0.22 and 0.44, 0.22.
 constexpr int kResLongSearch = 4096;
 constexpr int kHybLongSearch = 2048;
+
+// A search expands every arc of every vertex it reaches, the persistent kernel's
+// stops at a row's first hit: on dense graphs of the cluster's size that kernel
+// takes searches and phase 2.  Cut and phase 2, persistent and cluster: average
+// degree 60 (366k units) 0.14, 0.27 and 0.12, 0.22 ms, 120 (363k) 0.13, 0.17 and
+// 0.10, 0.25, 400 (401k) 0.10, 0.26 and 0.08, 0.19, 898 (405k) 0.08, 0.07 and 0.16,
+// 0.27; 400 (201k) 0.07, 0.06 and 0.19, 0.12, 76 (R-MAT, 159k) 0.09, 0.06 and 0.33,
+// 0.17; 30 (372k) 0.07, 0.07 and 0.27, 0.20.
+constexpr double kResDenseDegree = 50;
+constexpr long long kResDenseUnits = 1 << 18;
+// A wide search of few levels needs all SMs' bandwidth: on graphs of the hybrid
+// solver's size above so many units a search alone is the persistent kernel's where
+// the last solve's searches had fewer levels than this.  Cut, persistent and
+// hybrid: random graphs of 3.6M and 3.8M units (12 and 10 levels) 0.40, 0.63 and
+// 0.36, 0.63 ms, of 2.6M (9) 0.17, 0.11; grids of 3.6M (34) 0.61, 0.39, (174) 1.5,
+// 0.64; 3.5M (10, few vertices reached) 0.25, 0.16.
+constexpr long long kHybShallowUnits = 3600000;
+constexpr int kHybShallowLevels = 24;
 
 // Blocks for a graph of n vertices and na residual arcs: 1 where one block holds
 // it, kResMaxCluster where the cluster should (a row too long for its block's
