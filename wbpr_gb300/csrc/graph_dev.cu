@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cstdio>
 #include <cstring>
 #include <limits>
@@ -198,6 +199,9 @@ struct wbpr_graph {
   unsigned long long longest[3] = {0, 0, 0};
   int4* hyb_rec = nullptr;
   int levels = 0;                 // of a search in the last solve, on average
+  // of the solves and of phase 2: whether they start with a trial (trial_rounds)
+  enum Depth : char { kUnknown, kShallow, kDeep };
+  Depth depth[2] = {kUnknown, kUnknown};
   ResOut* res_out = nullptr;
   int64_t bytes = 0;
   std::vector<void*> allocs;
@@ -1848,6 +1852,26 @@ wbpr_status run_kernel(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch
   return WBPR_OK;
 }
 
+// Adds the counters of an earlier part of the same solve.
+void add_stats(Stats* s, const Stats& a) {
+  s->arcs_scanned += a.arcs_scanned;
+  s->pushes += a.pushes;
+  s->relabels += a.relabels;
+  s->vertex_visits += a.vertex_visits;
+  s->bfs_arcs += a.bfs_arcs;
+  s->bfs_vertices += a.bfs_vertices;
+  s->gr_ns += a.gr_ns;
+  s->round_ns += a.round_ns;
+  s->push_ns += a.push_ns;
+  s->heavy_visits += a.heavy_visits;
+  s->deep_ns += a.deep_ns;
+  s->deep_scanned += a.deep_scanned;
+  s->rounds += a.rounds;
+  s->grs += a.grs;
+  s->bfs_levels += a.bfs_levels;
+  s->bu_levels += a.bu_levels;
+}
+
 // Whether a launch goes to the resident or the hybrid solver.
 bool use_resident(const wbpr_graph* g, const RunCfg& rc) {
   if (!rc.resident || rc.term || (g->res_cluster == 0 && !g->hybrid)) return false;
@@ -1859,6 +1883,10 @@ bool use_resident(const wbpr_graph* g, const RunCfg& rc) {
   if (g->res_cluster) return row <= (search ? kResLongSearch : kResLongRow);
   if (search && g->levels < kHybShallowLevels) return row <= kHybLongSearch;
   return row <= (units > kHybLargeUnits ? kHybLongRowLarge : kHybLongRow);
+}
+
+bool few_rounds(const wbpr_graph* g, const Stats& s) {
+  return s.rounds <= trial_rounds(g->n + g->total_deg) && s.bfs_levels < kHybShallowLevels * std::max(1, s.grs);
 }
 
 // One launch of the resident or the hybrid solver.  *fits is cleared when
@@ -1920,6 +1948,8 @@ wbpr_status run_resident(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* laun
     g->res_cluster = g->res_cluster < kResMaxCluster ? kResMaxCluster : 0;
   }
   if (rc.mode != kModeBfsOnly) g->full_reset = true;  // its pushes are not in the undo log
+  if (rc.mode != kModeBfsOnly && h.err == 0 && !g->res_cluster && g->depth[rc.phase2] == g->kUnknown && few_rounds(g, h.st))
+    g->depth[rc.phase2] = g->kShallow;
   if (launch_ms) CK(cudaEventElapsedTime(launch_ms, g->ev2, g->ev3));
   g->trace_n = 0;
   *hs = h.st;
@@ -1928,16 +1958,54 @@ wbpr_status run_resident(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* laun
   return (wbpr_status)h.err;
 }
 
+// Whether a launch that use_resident() accepts starts with a trial on the
+// persistent kernel.
+bool starts_with_trial(const wbpr_graph* g, const RunCfg& rc) {
+  if (g->res_cluster || rc.mode == kModeBfsOnly || g->depth[rc.phase2] != g->kShallow) return false;
+  return g->n + g->total_deg >= (rc.phase2 ? kHybTrialPhase2 : kHybTrialUnits);
+}
+
 wbpr_status run_persistent(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch_ms) {
   return g->layout == WBPR_LAYOUT_RCSR ? run_kernel<TopoR>(g, rc, hs, launch_ms)
                                        : run_kernel<TopoB>(g, rc, hs, launch_ms);
 }
 
+// The trial, and what is left after it: the preflow and the residuals that the
+// persistent kernel leaves behind a round are a state like any other.
+wbpr_status run_trial(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch_ms) {
+  const auto t0 = std::chrono::steady_clock::now();
+  RunCfg first = rc;
+  first.max_rounds = trial_rounds(g->n + g->total_deg);
+  if (rc.max_rounds > 0 && rc.max_rounds <= first.max_rounds) first.max_rounds = rc.max_rounds;
+  float ms = 0;
+  wbpr_status st = run_persistent(g, first, hs, &ms);
+  if (launch_ms) *launch_ms = ms;
+  if (st == WBPR_OK && !few_rounds(g, *hs)) g->depth[rc.phase2] = g->kDeep;
+  if (st != WBPR_ERR_NO_CONVERGENCE || first.max_rounds == rc.max_rounds || hs->rounds < first.max_rounds) return st;
+  g->depth[rc.phase2] = g->kDeep;
+  RunCfg rest = rc;
+  rest.mode = kModeState;
+  if (rc.max_rounds > 0) rest.max_rounds -= hs->rounds;
+  const auto ns = std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now() - t0).count();
+  if ((unsigned long long)ns >= rc.budget_ns) return st;
+  rest.budget_ns -= (unsigned long long)ns;
+  const Stats done = *hs;
+  bool fits = false;
+  st = run_resident(g, rest, hs, &ms, nullptr, &fits);
+  if (!fits) st = run_persistent(g, rest, hs, &ms);
+  if (launch_ms) *launch_ms += ms;
+  add_stats(hs, done);
+  return st;
+}
+
 wbpr_status run(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* launch_ms = nullptr) {
-  if (rc.mode != kModeFresh && use_resident(g, rc)) {  // (a fresh solve has asked already)
-    bool fits = false;
-    const wbpr_status st = run_resident(g, rc, hs, launch_ms, nullptr, &fits);
-    if (st || fits) return st;
+  if (use_resident(g, rc)) {
+    if (starts_with_trial(g, rc)) return run_trial(g, rc, hs, launch_ms);
+    if (rc.mode != kModeFresh) {  // (a fresh solve has asked already)
+      bool fits = false;
+      const wbpr_status st = run_resident(g, rc, hs, launch_ms, nullptr, &fits);
+      if (st || fits) return st;
+    }
   }
   return run_persistent(g, rc, hs, launch_ms);
 }
@@ -2457,7 +2525,7 @@ wbpr_status wbpr_solve(wbpr_graph* g, int32_t s, int32_t t, wbpr_algo algo, cons
   float launch_ms = 0;
   int et = 0;
   bool done = false;  // by the resident solver, which starts from the capacities itself
-  if (!matched && use_resident(g, rc)) {
+  if (!matched && use_resident(g, rc) && !starts_with_trial(g, rc)) {
     st = run_resident(g, rc, &hs, &launch_ms, &et, &done);
     if (done) CK(cudaEventRecord(g->ev1, g->stream));
   }

@@ -123,6 +123,22 @@ cudaError_t launch_hybrid(const ResParams& p, cudaStream_t st);
 int hybrid_clusters(int blocks);
 cudaError_t launch_hybrid_batch(const ResBatch& b, int blocks, int clusters, cudaStream_t st);
 
+// The records' build and write-back are most of a hybrid solve of few rounds.
+// Once a handle's solve (or its phase 2) has ended there within trial_rounds()
+// and without deep searches, the next ones start on the persistent kernel, for so
+// many rounds; one that has not ended by then goes over to the hybrid solver with
+// the preflow it has, and so do all that follow.  (A trial in a handle's first
+// solve too would take 0.44 ms of the 0.67 below, but 1.8 of 0.9 where 76 rounds
+// follow.)  A round costs about 14 us more on the persistent kernel; what is saved
+// is 0.03 to 0.07 ms per million vertices and residual arcs.  First and next call on
+// a handle, persistent kernel alone and by this rule: random graphs of 3.6M units,
+// 13 rounds 0.43, 0.42 and 0.67, 0.45 ms; of 2.5M, no way to t, RCSR 0.08, 0.08 and
+// 0.20, 0.09; phase 2 of a 512x512 grid 0.32, 0.29 and 0.51, 0.32, of random graphs
+// of 3.8M 0.22, 0.21 and 0.68, 0.23.
+constexpr long long kHybTrialUnits = 1 << 18;
+constexpr long long kHybTrialPhase2 = 1 << 20;  // below, the hybrid solver is never the slower one
+inline long long trial_rounds(long long units) { return units >> 18; }
+
 // Above this many vertices and residual arcs a graph that both could take goes
 // to the hybrid solver: its vertices are dealt to the blocks one by one, the
 // resident solver's in runs.  GENRMF 16x40 (107k units) 3.9 ms resident, 4.7
