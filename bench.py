@@ -635,8 +635,8 @@ def load_pins() -> dict:
 
 
 def batch_record(count: int, steps: int, warmup: int, loop_sample: int = 96, union: bool = False) -> dict:
-    """Config 3: `count` uneven instances in one persistent launch (CUDA graph
-    replay, tuning from wbpr_batch_autotune), every flow checked against the
+    """Config 3: `count` uneven instances in one batch (a CUDA graph of concurrent
+    launches, tuning from wbpr_batch_autotune), every flow checked against the
     oracle's pinned values, against a loop of the plain single-instance
     solver over a seeded sample of the same instances."""
     import numpy as np
@@ -747,7 +747,7 @@ def adjoint_record(grids: int, warmup: int, fd_arcs: int = 0) -> dict:
 
 
 def config3(args):
-    """4,096 uneven instances in one persistent launch (CUDA graph replay,
+    """4,096 uneven instances in one batch (a CUDA graph of concurrent launches,
     autotuned) against a loop of the plain solver over a sample.  Under
     torchrun the instances are sharded across the ranks by estimated work
     (wbpr_gb300.shard), one batched launch per rank, and the flows gathered

@@ -325,8 +325,9 @@ wbpr_status wbpr_solve_pairs(wbpr_graph* g, int32_t k, const int32_t* sources, c
  * with bfs_alpha 4, gr_plateau 4 and both; return the fastest tuning and its
  * solve time.  On a graph that a shared-memory solver takes and solves faster
  * than the persistent kernel does with the best of its knobs, the tuning
- * returned has those knobs and resident = 1.  Every tuning must give the same flow (WBPR_ERR_VERIFY
- * otherwise).  The graph's state afterwards is that of the last solve. */
+ * returned has those knobs and resident = 1.  Every tuning must give the same
+ * flow (WBPR_ERR_VERIFY otherwise).  The graph's state afterwards is that of
+ * the last solve. */
 wbpr_status wbpr_autotune(wbpr_graph* g, int32_t s, int32_t t, wbpr_algo algo, wbpr_tuning* best,
                           float* best_ms);
 /* Read back the state after a solve (host buffers, any may be NULL):
@@ -384,8 +385,9 @@ wbpr_status wbpr_batch_solve(wbpr_batch* b, const wbpr_tuning* tuning, int64_t* 
 /* Per-instance device time (ms) and rounds of the last solve (either may be NULL). */
 wbpr_status wbpr_batch_instance_stats(wbpr_batch* b, float* inst_ms, int32_t* inst_rounds);
 /* Try tile widths, block sizes and global-relabel frequencies on this batch,
- * then which instances run on clusters (batch_cluster: none, 2^18 or 2^19
- * units); return the fastest tuning and its time. */
+ * then other splits (batch_cluster: -1, 2^18 or 2^19 units) on the best of
+ * those; return the fastest tuning and its time.  The defaults, which the
+ * shared-memory solvers take part in, are among them. */
 wbpr_status wbpr_batch_autotune(wbpr_batch* b, wbpr_tuning* best, float* best_ms);
 
 /* ---- solve without any device allocation --------------------------------- */

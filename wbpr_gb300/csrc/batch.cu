@@ -456,7 +456,9 @@ int hybrid_class(int64_t n, int64_t units, double t, int least) {
 //   21 instances 68 -> 8.3 ms, 100 122 -> 13 ms, 512 295 -> 38 ms, 2,048
 //   331 -> 88 ms, 4,096 361 -> 160 ms (p99 of an instance 155 -> 40 ms).
 // With every instance from 2^16 or 2^17 units on 16 blocks 512 take 92 and 70
-// ms, with none 68 ms.
+// ms, with none 68 ms.  (All launches are concurrent: three GENRMF 30x44 on clusters
+// and an instance on a block take 19.7 and 37.4 ms alone and 36.6 together, with
+// tile 32 83, 49 and 79.)
 wbpr_status capture(wbpr_batch* b, int tile, int block, double alpha, int grr, long long max_rounds,
                     double max_ms, int64_t cluster_units, bool mixed) {
   if (b->exec && b->cap_tile == tile && b->cap_block == block && b->cap_alpha == alpha && b->cap_grr == grr &&
@@ -879,8 +881,10 @@ wbpr_status wbpr_batch_autotune(wbpr_batch* b, wbpr_tuning* best, float* best_ms
           bt = t;
         }
       }
-  // then, on the best of those, which instances get clusters: none, or
-  // from 2^18 or 2^19 units instead of 3 x 2^17
+  // then, on the best of those, other splits than its own (the defaults: a class
+  // an instance; with a knob set, clusters from 3 x 2^17 units): the general kernel
+  // without clusters, or clusters from 2^18 or 2^19 units (with the defaults, the
+  // hybrid solver's largest from there on and its smallest below)
   const int64_t cls[] = {-1, 1 << 18, 1 << 19};
   if (bms < 1e29f)
     for (int64_t c : cls) {

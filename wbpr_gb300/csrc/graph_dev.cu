@@ -1933,7 +1933,7 @@ wbpr_status run_resident(wbpr_graph* g, const RunCfg& rc, Stats* hs, float* laun
     p.run.budget_ns = rc.budget_ns;
     p.keep = true;
     p.rec = g->hyb_rec;
-    const cudaError_t e = g->res_cluster ? launch_resident(p, g->avg_deg < 20 ? 8 : 32, g->res_cluster, g->stream)
+    const cudaError_t e = g->res_cluster ? launch_resident(p, g->avg_deg < kResWideDegree ? 8 : 32, g->res_cluster, g->stream)
                                          : launch_hybrid(p, g->stream);
     if (e != cudaSuccess) {
       cudaGetLastError();  // no such cluster on this device: the persistent kernel takes the graph

@@ -306,7 +306,7 @@ extern "C" wbpr_status wbpr_solve_bcsr_noalloc(int32_t n, int64_t num_residual_a
     rp.run.budget_ns = 120ull * 1000 * 1000 * 1000;
     rp.gate = counts + 8;
     rp.keep = true;
-    const cudaError_t launched = launch_resident(rp, num_residual_arcs < 20LL * n ? 8 : 32, cluster, st);
+    const cudaError_t launched = launch_resident(rp, num_residual_arcs < (long long)kResWideDegree * n ? 8 : 32, cluster, st);
     if (launched != cudaSuccess) cudaGetLastError();  // no such cluster on this device: as below
     NA_CK(cudaMemcpyAsync(&h.out, out, sizeof(h.out), cudaMemcpyDeviceToHost, st));
     NA_CK(cudaMemcpyAsync(h.counts, counts, sizeof(h.counts), cudaMemcpyDeviceToHost, st));

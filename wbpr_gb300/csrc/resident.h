@@ -186,6 +186,16 @@ constexpr long long kResDenseUnits = 1 << 18;
 constexpr long long kHybShallowUnits = 3600000;
 constexpr int kHybShallowLevels = 24;
 
+// Lanes of a row in the resident solver: 8 below this average degree, 32 from it
+// on.  Means of four seeds, 8 and 32 lanes: random graphs of 1,000 vertices, degree
+// 8 0.081, 0.094 ms, 18 0.102, 0.111, 22 0.083, 0.089, 28 0.112, 0.107, 40 0.127,
+// 0.113, 80 0.144, 0.113; of 3,000 8 0.166, 0.170, 18 0.136, 0.130, 28 0.178, 0.171,
+// 80 0.291, 0.251; R-MAT scale 11 to 13 7 0.264, 0.296; 0.200, 0.175; 0.262, 0.229, 14
+// 0.181, 0.161; 0.235, 0.223; 0.370, 0.323, 20 0.199, 0.188; 0.291, 0.269; 0.421,
+// 0.396, 27 0.228, 0.206; 0.338, 0.310; 0.505, 0.473.  (Batches have one kernel, of 8
+// lanes: most of their instances are sparse.)
+constexpr int kResWideDegree = 20;
+
 // Blocks for a graph of n vertices and na residual arcs: 1 where one block holds
 // it, kResMaxCluster where the cluster should (a row too long for its block's
 // share can still keep it out), or 0.
