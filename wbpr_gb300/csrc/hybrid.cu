@@ -21,12 +21,12 @@
 // access an arc (grid 512x512 37 -> 34 ms).
 //
 // Measured on GB300, persistent kernel and now:
-//   GENRMF 32x64 (65,536 vertices)     183  -> 30 ms
+//   GENRMF 32x64 (65,536 vertices)     183  -> 24 ms (mean of ten seeds)
 //   GENRMF 40x80 (128,000 vertices)    230  -> 48 ms
 //   grid 512x512 (three seeds)         45, 44, 21 -> 17, 17, 10-13 ms
 //   grid 200x200                       27.3 -> 6.0 ms
 //   layered 100x2500 (250,002)         14.6 -> 3.8-4.8 ms
-//   layered 64x512                     6.1  -> 1.0-1.1 ms (2.0 ms resident)
+//   layered 64x512                     6.1  -> 1.1 ms (2.0 ms resident)
 // What bounds it: the chain of a step, and on the largest graphs the 16 SMs.
 #include "resident.cuh"
 

@@ -14,13 +14,14 @@
 // returning atomic.  A step pushes and relabels in one pass (discharge()), so
 // a round has one barrier instead of two.
 //
-// Measured on GB300, solve time before (persistent kernel) and now:
-//   GENRMF 4x5 (80 vertices, one block)            1.00 -> 0.13 ms
-//   GENRMF 8x16 (1,024 vertices, one block), RCSR  7.69 -> 0.58 ms
-//   layered 11x37 (409 vertices, one block), RCSR  1.91 -> 0.14 ms
-//   GENRMF 16x40 (10,240 vertices, cluster)        33.8 -> 3.74 ms
-//   layered 32x256 (8,194 vertices, cluster)       2.96 -> 0.53 ms
-//   R-MAT scale 13 (221k residual arcs, cluster)   0.70 -> 0.47 ms
+// Measured on GB300, solve time before (persistent kernel, one seed) and now (mean
+// of ten seeds where the families' names say no more):
+//   GENRMF 4x5 (80 vertices, one block)            1.00 -> 0.11 ms
+//   GENRMF 8x16 (1,024 vertices, one block), RCSR  7.69 -> 0.69 ms
+//   layered 11x37 (409 vertices, one block), RCSR  1.91 -> 0.13 ms
+//   GENRMF 16x40 (10,240 vertices, cluster)        33.8 -> 3.9 ms (one seed)
+//   layered 32x256 (8,194 vertices, cluster)       2.96 -> 0.75 ms (one seed)
+//   R-MAT scale 13 (230k residual arcs, cluster)   0.70 -> 0.48 ms, RCSR 0.78 -> 0.51
 // A round takes 1.0-1.7 us in one block and about 2.2 us in the cluster, a BFS
 // level 0.6-0.8 us in one block; what bounds it now is the length of one
 // warp's instruction chain through discharge() (about 1,000 cycles) and, in
