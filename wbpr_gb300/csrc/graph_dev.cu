@@ -1024,8 +1024,10 @@ __global__ void db_cls_scatter(const int* o1, const int* o2, int n, const int* s
     else cls[n01 + s2[u]] = u;
   }
 }
-// the three longest of nh heavy rows, arcs << 32 | vertex, longest first (0: none); one block
-__global__ void db_longest(const int* o1, const int* o2, const int* hcls, int nh, unsigned long long* out) {
+// the three longest of nh heavy rows, arcs << 32 | vertex, longest first (0: none),
+// and the number of their chunks; one block
+__global__ void db_longest(const int* o1, const int* o2, const int* hcls, int nh, const int* nch, unsigned long long* out) {
+  if (threadIdx.x == 0) out[3] = (unsigned long long)nch[nh];
   __shared__ unsigned long long best;
   unsigned long long below = ~0ull;
   for (int k = 0; k < 3; ++k) {
@@ -1402,8 +1404,19 @@ wbpr_status build_device(wbpr_graph* g, const wbpr_csr* in) {
   DB(cudaGetLastError());
   DBS(device_scan(cbase, (long long)nh + 1, st));
   int nbch = 0;
-  DB(cudaMemcpyAsync(&nbch, cbase + nh, 4, cudaMemcpyDeviceToHost, st));
-  DB(cudaStreamSynchronize(st));
+  if (nh > 0 && (g->n + g->total_deg <= kHybMaxUnits || g->n_td_heavy < kFewLong)) {
+    // a graph that a shared-memory solver may take, or one with few long rows
+    unsigned long long heavy[4];
+    db_longest<<<1, 256, 0, st>>>(o1, o2, hcls, nh, cbase, cnt);  // the counters have been read
+    DB(cudaGetLastError());
+    DB(cudaMemcpyAsync(heavy, cnt, sizeof(heavy), cudaMemcpyDeviceToHost, st));
+    DB(cudaStreamSynchronize(st));
+    for (int k = 0; k < 3; ++k) g->longest[k] = heavy[k];
+    nbch = (int)heavy[3];
+  } else if (nh > 0) {
+    DB(cudaMemcpyAsync(&nbch, cbase + nh, 4, cudaMemcpyDeviceToHost, st));
+    DB(cudaStreamSynchronize(st));
+  }
   g->n_bch = nbch;
   DBS(dalloc(g, &g->bch, (size_t)nbch));
   if (nh) db_bch_fill<<<std::min(nh, blocks), 128, 0, st>>>(o1, o2, hcls, nh, cbase, g->bch);
@@ -1593,15 +1606,6 @@ wbpr_status build_on_device(wbpr_graph* g, const wbpr_csr* in) {
     CK(cudaMemsetAsync(g->ulog_n, 0, sizeof(int) * (size_t)kLogSlots * kLogStride, g->stream));
   }
   // in the stream the pool allocations were made on (stream-ordered memory)
-  // a graph that a shared-memory solver may take, or one with few long rows
-  if (g->n_heavy > 0 && (g->n + g->total_deg <= kHybMaxUnits || g->n_td_heavy < kFewLong)) {
-    auto* three = (unsigned long long*)g->h;  // 64 words at least, cleared below
-    const bool bcsr = g->layout == WBPR_LAYOUT_BCSR;
-    db_longest<<<1, 256, 0, g->stream>>>(bcsr ? g->row : g->frow, bcsr ? nullptr : g->rrow, g->cls + g->n_light + g->n_medium,
-                                         g->n_heavy, three);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(g->longest, three, sizeof(g->longest), cudaMemcpyDeviceToHost, g->stream));
-  }
   CK(cudaMemsetAsync(g->h, 0, 4 * (size_t)g->n, g->stream));
   CK(cudaMemsetAsync(g->e, 0, 4 * (size_t)g->n, g->stream));
   CK(cudaStreamSynchronize(g->stream));
